@@ -24,10 +24,10 @@ _ip = np.ctypeslib.ndpointer(dtype=np.int32, flags="C_CONTIGUOUS")
 
 def reference_dir() -> str | None:
     """Where LAP's sources are mounted: $LAP_REFERENCE_DIR, else the default
-    mount point of this build's container; None where neither exists (the
-    GPU hosts, which only run the prebuilt oracle)."""
+    mount point; None where that holds no sources (hosts that only run the
+    oracle)."""
     d = os.environ.get("LAP_REFERENCE_DIR") or "/root/reference"
-    return d if os.path.isdir(d) else None
+    return d if os.path.isfile(os.path.join(d, "cg.c")) else None
 
 
 def build(ref_dir: str | None = None, quiet: bool = True) -> None:
