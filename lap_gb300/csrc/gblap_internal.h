@@ -74,7 +74,32 @@ struct RecordSet {
   void *long_val = nullptr;      // [nlong] values of long rows
 };
 
+// Lock-step form of a factor (tri_step.h): built for factors whose rows have
+// few, near dependencies; the PCG's solves then run it instead of the records.
+struct StepPlan {
+  bool on = false;
+  int elem = 0;       // bytes of a value: 4 or 8
+  int k = 0;          // the most dependencies a row has (2, 3 or 4)
+  int ntiles = 0, tile_rows = 0;
+  int nw = 0;         // solver warps
+  int np = 0;         // staged pages
+  int window = 0;     // places of the tile's own values (a power of two)
+  int nexp_max = 0;   // inbox places
+  int cluster = 1, ngroups = 0;
+  int max_steps = 0;
+  long long npages = 0;
+  size_t smem = 0;
+  void *tiles = nullptr;             // StepTile [ntiles]
+  unsigned short *ends = nullptr;    // end position of each step
+  unsigned char *pages = nullptr;    // [npages] row data in step order
+  int *psrc = nullptr;               // [npages * kStepPage * 4] value source of each coefficient or -1
+  int *pdiag = nullptr;              // [npages * kStepPage] diagonal source or -1
+  void *mail = nullptr;              // [ngroups][nexp_max]
+  unsigned *ticket = nullptr;
+};
+
 struct TriPlan {
+  StepPlan step;
   int n = 0;
   bool lower = true;
   int nlevels = 0;           // global dependency depth (diagnostics)

@@ -27,6 +27,7 @@
 #include "pcg.h"
 #include "pcg_state.cuh"
 #include "sptrsv.h"
+#include "tri_step.h"
 #include "system.h"
 
 namespace gb {
@@ -264,6 +265,26 @@ __global__ void __launch_bounds__(kThreads)
     for (int u = 0; u < kEwUnroll; ++u) acc[0] = fma((double)rv[u], (double)wv[u], acc[0]);
   }
   for (; i < n; i += stride) acc[0] = fma((double)r[i], (double)w[i], acc[0]);
+  if (reduce_last<1>(acc, part, gridDim.x, blockIdx.x, &st->tk[TK_RHO], sm) && threadIdx.x == 0) {
+    st->rho_prev = st->rho;
+    st->rho = acc[0];
+  }
+}
+
+// GS_std after its backward sweep in lock-step form: w = t + y (GS.c:39-40)
+// and r'w in one pass; rho_prev <- rho.
+template <typename T, typename TW>
+__global__ void __launch_bounds__(kThreads)
+    rho_add_kernel(int n, const T* __restrict__ r, const TW* __restrict__ t, const TW* __restrict__ y,
+                   TW* __restrict__ w, PcgState* st, double* part) {
+  __shared__ double sm[kThreads / 32];
+  if (st->done) return;
+  double acc[1] = {0.0};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const TW wv = t[i] + y[i];
+    w[i] = wv;
+    acc[0] = fma((double)r[i], (double)wv, acc[0]);
+  }
   if (reduce_last<1>(acc, part, gridDim.x, blockIdx.x, &st->tk[TK_RHO], sm) && threadIdx.x == 0) {
     st->rho_prev = st->rho;
     st->rho = acc[0];
@@ -633,6 +654,7 @@ static int launch_lower(gb_system sys, PcgState* st, int do_update, cudaGraphCon
     GB_CUDA_TRY(cudaGetLastError());
   }
   const TriPlan& L = sizeof(T) == 8 ? sys->L : sys->L32;
+  if (L.step.on) return step_solve<T, T>(L.step, v.r, v.t, &st->done, sys->err, sys->s);
   OpSplitLower<T, T> op{v.r, v.s, st, false};
   return tri_launch<T, OpSplitLower<T, T>, false>(L, tri_args<T>(L, v.t, sys->err, true), op, sys->s);
 }
@@ -642,9 +664,16 @@ template <typename T>
 static int launch_upper(gb_system sys, PcgState* st) {
   auto v = vecs<T>(sys);
   const TriPlan& U = sizeof(T) == 8 ? sys->U : sys->U32;
+  const TriPlan& L = sizeof(T) == 8 ? sys->L : sys->L32;
+  // a record-form lower solve leaves the sentinel in s; the lock-step one does not
+  if (L.step.on && !U.step.on) GB_TRY(fill_sentinel_dev(sys->n, v.s, sys->s));
   if (sys->prec == GB_PREC_ICHOL) {
-    OpSplitUpper<T> op{v.t, st, false};
-    GB_TRY((tri_launch<T, OpSplitUpper<T>, false>(U, tri_args<T>(U, v.s, sys->err, true), op, sys->s)));
+    if (U.step.on) {
+      GB_TRY((step_solve<T, T>(U.step, v.t, v.s, &st->done, sys->err, sys->s)));
+    } else {
+      OpSplitUpper<T> op{v.t, st, false};
+      GB_TRY((tri_launch<T, OpSplitUpper<T>, false>(U, tri_args<T>(U, v.s, sys->err, true), op, sys->s)));
+    }
     rho_kernel<T><<<grid_ew(sys->n), kThreads, 0, sys->s>>>(sys->n, v.r, v.s, st, sys->part);
     GB_CUDA_TRY(cudaGetLastError());
     return GB_OK;
@@ -654,6 +683,12 @@ static int launch_upper(gb_system sys, PcgState* st) {
                         sys->s>>>(sys->n, nb, sys->plan.bundles, sys->ia, sys->ja, mat_vals<T>(sys), v.t, v.r,
                                   v.p1, st);
   GB_CUDA_TRY(cudaGetLastError());
+  if (U.step.on) {
+    GB_TRY((step_solve<T, T>(U.step, v.p1, v.s, &st->done, sys->err, sys->s)));
+    rho_add_kernel<T, T><<<grid_ew(sys->n), kThreads, 0, sys->s>>>(sys->n, v.r, v.t, v.s, v.w, st, sys->part);
+    GB_CUDA_TRY(cudaGetLastError());
+    return GB_OK;
+  }
   OpSplitGsUpper<T> op{v.p1, v.t, v.w, st, false};
   GB_TRY((tri_launch<T, OpSplitGsUpper<T>, false>(U, tri_args<T>(U, v.s, sys->err, true), op, sys->s)));
   rho_kernel<T><<<grid_ew(sys->n), kThreads, 0, sys->s>>>(sys->n, v.r, v.w, st, sys->part);
@@ -676,6 +711,7 @@ int launch_prologue(gb_system sys, PcgState* st, int x_zero, const T* b) {
   auto v = vecs<T>(sys);
   const int wk = prec_wkind(sys->prec, sys->k);
   const bool tri = prec_fused_tri(sys->prec, sys->k);
+  const bool step = (sizeof(T) == 8 ? sys->L : sys->L32).step.on;  // needs no sentinel in t
   const int nb = sys->plan.nbundles;
   const int g = grid_for_bundles<T>(nb);
   const T* a = mat_vals<T>(sys);
@@ -683,7 +719,7 @@ int launch_prologue(gb_system sys, PcgState* st, int x_zero, const T* b) {
 #define GB_RESID(WKV)                                                                          \
   resid_kernel<T, WKV><<<g, kThreads, 0, sys->s>>>(sys->n, nb, sys->plan.bundles, sys->ia,     \
                                                    sys->ja, a, b, v.x, x_zero, v.r, v.w, dr,    \
-                                                   tri ? v.t : nullptr, st, sys->part, sys->hist)
+                                                   tri && !step ? v.t : nullptr, st, sys->part, sys->hist)
   if (wk == WK_NONE) GB_RESID(WK_NONE);
   else if (wk == WK_JACOBI) GB_RESID(WK_JACOBI);
   else GB_RESID(WK_PREC);
@@ -709,16 +745,24 @@ int launch_prologue(gb_system sys, PcgState* st, int x_zero, const T* b) {
 // preconditioner: the triangular solves run on the FMA-form FP32 records
 // with FP32 outputs t (lower) and s / w (upper).
 static int launch_lower_split(gb_system sys, PcgState* st) {
+  if (sys->L32.step.on)
+    return step_solve<float, double>(sys->L32.step, sys->v64.r, sys->v32.t, &st->done, sys->err, sys->s);
   OpSplitLower<float, double> op{sys->v64.r, sys->v32.s, st, false};
   return tri_launch<float, OpSplitLower<float, double>, false>(
       sys->L32, tri_args<float>(sys->L32, sys->v32.t, sys->err, true), op, sys->s);
 }
 
 static int launch_upper_split(gb_system sys, PcgState* st) {
+  const bool step = sys->U32.step.on;
+  if (sys->L32.step.on && !step) GB_TRY(fill_sentinel_dev(sys->n, sys->v32.s, sys->s));
   if (sys->prec == GB_PREC_ICHOL) {
-    OpSplitUpper<float> op{sys->v32.t, st, false};
-    GB_TRY((tri_launch<float, OpSplitUpper<float>, false>(
-        sys->U32, tri_args<float>(sys->U32, sys->v32.s, sys->err, true), op, sys->s)));
+    if (step) {
+      GB_TRY((step_solve<float, float>(sys->U32.step, sys->v32.t, sys->v32.s, &st->done, sys->err, sys->s)));
+    } else {
+      OpSplitUpper<float> op{sys->v32.t, st, false};
+      GB_TRY((tri_launch<float, OpSplitUpper<float>, false>(
+          sys->U32, tri_args<float>(sys->U32, sys->v32.s, sys->err, true), op, sys->s)));
+    }
     rho_kernel<double, float><<<grid_ew(sys->n), kThreads, 0, sys->s>>>(sys->n, sys->v64.r, sys->v32.s,
                                                                         st, sys->part);
     GB_CUDA_TRY(cudaGetLastError());
@@ -731,6 +775,13 @@ static int launch_upper_split(gb_system sys, PcgState* st) {
                                  kThreads, 0, sys->s>>>(sys->n, nb, sys->plan.bundles, sys->ia, sys->ja,
                                                         sys->a32, sys->v32.t, sys->v64.r, sys->v32.r, st);
   GB_CUDA_TRY(cudaGetLastError());
+  if (step) {
+    GB_TRY((step_solve<float, float>(sys->U32.step, sys->v32.r, sys->v32.s, &st->done, sys->err, sys->s)));
+    rho_add_kernel<double, float><<<grid_ew(sys->n), kThreads, 0, sys->s>>>(sys->n, sys->v64.r, sys->v32.t,
+                                                                            sys->v32.s, sys->v32.w, st, sys->part);
+    GB_CUDA_TRY(cudaGetLastError());
+    return GB_OK;
+  }
   OpSplitGsUpper<float> op{sys->v32.r, sys->v32.t, sys->v32.w, st, false};
   GB_TRY((tri_launch<float, OpSplitGsUpper<float>, false>(
       sys->U32, tri_args<float>(sys->U32, sys->v32.s, sys->err, true), op, sys->s)));
@@ -747,7 +798,7 @@ static int grid_split(int nb) {
 // w = M^-1 r for the current FP64 r (the lower solve's output is pre-filled
 // with the sentinel first); the upper solve rolls rho.
 static int apply_prec_split(gb_system sys, PcgState* st) {
-  GB_TRY(fill_sentinel_dev(sys->n, sys->v32.t, sys->s));
+  if (!sys->L32.step.on) GB_TRY(fill_sentinel_dev(sys->n, sys->v32.t, sys->s));
   GB_TRY(launch_lower_split(sys, st));
   return launch_upper_split(sys, st);
 }
@@ -768,7 +819,8 @@ int launch_body_split(gb_system sys, PcgState* st, cudaGraphConditionalHandle co
   const int nb = sys->plan.nbundles;
   const float* w = sys->prec == GB_PREC_ICHOL ? sys->v32.s : sys->v32.w;
   spmv_pq_split_kernel<<<grid_split(nb), kThreads, 0, sys->s>>>(
-      sys->n, nb, sys->plan.bundles, sys->ia, sys->ja, sys->a32, w, v.p0, v.q, sys->v32.t, st,
+      sys->n, nb, sys->plan.bundles, sys->ia, sys->ja, sys->a32, w, v.p0, v.q,
+      sys->L32.step.on ? nullptr : sys->v32.t, st,
       sys->part, cond, has_cond);
   GB_CUDA_TRY(cudaGetLastError());
   const double n = sys->n, nz = sys->nnz;
@@ -807,6 +859,7 @@ int launch_body(gb_system sys, PcgState* st, cudaGraphConditionalHandle cond, in
   auto v = vecs<T>(sys);
   const int wk = prec_wkind(sys->prec, sys->k);
   const bool tri = prec_fused_tri(sys->prec, sys->k);
+  const bool step = (sizeof(T) == 8 ? sys->L : sys->L32).step.on;  // needs no sentinel in t
   const int nb = sys->plan.nbundles;
   const int g = grid_for_bundles<T>(nb);
   const T* a = mat_vals<T>(sys);
@@ -815,7 +868,7 @@ int launch_body(gb_system sys, PcgState* st, cudaGraphConditionalHandle cond, in
 #define GB_PQ(WKV)                                                                             \
   spmv_pq_kernel<T, WKV><<<g, kThreads, 0, sys->s>>>(sys->n, nb, sys->plan.bundles, sys->ia,   \
                                                      sys->ja, a, wbuf, v.p0, v.q,               \
-                                                     tri ? v.t : nullptr, st, sys->part, cond,  \
+                                                     tri && !step ? v.t : nullptr, st, sys->part, cond,  \
                                                      has_cond)
   if (wk == WK_NONE) GB_PQ(WK_NONE);
   else if (wk == WK_JACOBI) GB_PQ(WK_JACOBI);
@@ -903,7 +956,7 @@ int launch_resume(gb_system sys, PcgState* st, double delta) {
     // w = M^-1 r for the replaced r; the upper solve rolls rho.  The lower
     // solve's output still holds the last solve's values: refill it with the
     // sentinel, or later tiles would read them as finished.
-    GB_TRY(fill_sentinel_dev(sys->n, v.t, sys->s));
+    if (!(sizeof(T) == 8 ? sys->L : sys->L32).step.on) GB_TRY(fill_sentinel_dev(sys->n, v.t, sys->s));
     GB_TRY(launch_lower<T>(sys, st, 0, 0, 0));
     return launch_upper<T>(sys, st);
   }

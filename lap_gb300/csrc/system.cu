@@ -18,6 +18,7 @@
 #include "pcg.h"
 #include "pcg_state.cuh"
 #include "sptrsv.h"
+#include "tri_step.h"
 #include "system.h"
 
 using namespace gb;
@@ -315,24 +316,25 @@ extern "C" int gb_system_create(int n, int nnz, const int* ia, const int* ja, co
     // GBLAP_TRI_TILE_ROWS32 sets both explicitly.
     const int t32l = tri_default_tile_rows32(n);
     const int t32u = t32l;
-    // The four plans are independent host work (levels, record packing,
-    // layout): built on parallel threads, each with this thread's device
-    // current (4.19M-row Chung-Lu: 8.8 s one after another).
+    // The plans are independent host work (levels, packing, layout), built on
+    // parallel threads, each with this thread's device current (4.19M-row
+    // Chung-Lu: 8.8 s one after another).  An FP64 factor has two: the exact
+    // solves' records and, where the factor allows it, the lock-step form.
     {
       int dev = 0;
       CKC(cudaGetDevice(&dev));
       (void)device_sm_count();  // initialised once here, read by the workers
       const int w32 = tri_consumer_warps(4);
-      int rcs[4] = {GB_OK, GB_OK, GB_OK, GB_OK};
-      std::thread th[4] = {
-          std::thread([&] { rcs[0] = cudaSetDevice(dev) == cudaSuccess ? tri_plan_build(dl, &s->L) : GB_CUDA_ERROR; }),
-          std::thread([&] { rcs[1] = cudaSetDevice(dev) == cudaSuccess ? tri_plan_build(du, &s->U) : GB_CUDA_ERROR; }),
-          std::thread([&] {
-            rcs[2] = cudaSetDevice(dev) == cudaSuccess ? tri_plan_build(dl, &s->L32, t32l, w32) : GB_CUDA_ERROR;
-          }),
-          std::thread([&] {
-            rcs[3] = cudaSetDevice(dev) == cudaSuccess ? tri_plan_build(du, &s->U32, t32u, w32) : GB_CUDA_ERROR;
-          })};
+      int rcs[6] = {GB_OK, GB_OK, GB_OK, GB_OK, GB_OK, GB_OK};
+      auto on_device = [dev](int* rc, auto build) {
+        return std::thread([=] { *rc = cudaSetDevice(dev) == cudaSuccess ? build() : (int)GB_CUDA_ERROR; });
+      };
+      std::thread th[6] = {on_device(&rcs[0], [&] { return tri_plan_build(dl, &s->L); }),
+                           on_device(&rcs[1], [&] { return tri_plan_build(du, &s->U); }),
+                           on_device(&rcs[2], [&] { return tri_step_plan_build(dl, &s->L, 8); }),
+                           on_device(&rcs[3], [&] { return tri_step_plan_build(du, &s->U, 8); }),
+                           on_device(&rcs[4], [&] { return tri_plan_build_fp32(dl, &s->L32, t32l, w32); }),
+                           on_device(&rcs[5], [&] { return tri_plan_build_fp32(du, &s->U32, t32u, w32); })};
       for (auto& t : th) t.join();
       for (int r : rcs) CK(r);
     }
@@ -625,6 +627,8 @@ static int solve_internal(gb_system s, const gb_pcg_opts* oin, gb_pcg_result* re
   const gb_pcg_opts* o = &oc;
   GB_TRY(system_ensure_hist(s, o->maxit));
   GB_CUDA_TRY(cudaMemsetAsync(s->err, 0, sizeof(int), s->s));
+  for (TriPlan* p : {o->precision == 0 ? &s->L : &s->L32, o->precision == 0 ? &s->U : &s->U32})
+    GB_TRY(step_plan_reset(&p->step, s->s));
   gb_pcg_result r;
   memset(&r, 0, sizeof r);
   PcgState* hs = s->st_host;

@@ -9,6 +9,7 @@
 #include "kernels.h"
 #include "sptrsv.h"
 #include "tri_kernel.cuh"
+#include "tri_step.h"
 
 namespace gb {
 
@@ -186,6 +187,52 @@ void free_set(RecordSet* rs) {
 
 }  // namespace
 
+// A record form asked for through its own settings keeps the records.
+static bool record_form_forced() {
+  for (const char* e : {"GBLAP_TRI_FORM", "GBLAP_TRI_SHORT", "GBLAP_TRI_FIXED", "GBLAP_TRI_CLUSTER",
+                        "GBLAP_TRI_FP64_CLUSTER", "GBLAP_TRI_TILE_ROWS", "GBLAP_TRI_TILE_ROWS32",
+                        "GBLAP_TRI_BLOCKS_PER_SM"})
+    if (getenv(e)) return true;
+  return false;
+}
+
+// Global levels (dependency depth) of the rows; returns their number.
+static int row_levels(const TriDeps& d, std::vector<int>* out) {
+  const int n = d.n;
+  std::vector<int>& lev = *out;
+  lev.assign(n, 0);
+  int nlev = 0;
+  for (int q = 0; q < n; ++q) {
+    const int i = d.lower ? q : n - 1 - q;
+    int l = 0;
+    for (int k = d.row_ptr[i]; k < d.row_ptr[i + 1]; ++k) l = std::max(l, lev[d.dep_col[k]] + 1);
+    lev[i] = l;
+    nlev = std::max(nlev, l + 1);
+  }
+  return nlev;
+}
+
+int tri_step_plan_build(const TriDeps& d, TriPlan* plan, int elem) {
+  if (record_form_forced()) return GB_OK;
+  std::vector<int> lev;
+  const int nlev = row_levels(d, &lev);
+  GB_TRY(step_plan_build(d, lev, nlev, elem, &plan->step));
+  if (plan->step.on && elem == 4) {  // nothing else reads this plan
+    plan->n = d.n;
+    plan->lower = d.lower;
+    plan->nlevels = nlev;
+    plan->ntiles = plan->step.ntiles;
+    plan->tile_rows = plan->step.tile_rows;
+    plan->ndeps = (long long)d.dep_col.size();
+  }
+  return GB_OK;
+}
+
+int tri_plan_build_fp32(const TriDeps& d, TriPlan* plan, int tile_rows, int level_run) {
+  GB_TRY(tri_step_plan_build(d, plan, 4));
+  return plan->step.on ? GB_OK : tri_plan_build(d, plan, tile_rows, level_run);
+}
+
 int tri_plan_build(const TriDeps& d, TriPlan* plan, int tile_rows, int level_run) {
   const int n = d.n;
   const bool lower = d.lower;
@@ -194,15 +241,8 @@ int tri_plan_build(const TriDeps& d, TriPlan* plan, int tile_rows, int level_run
   auto deps_of = [&](int r) { return d.row_ptr[r + 1] - d.row_ptr[r]; };
 
   // global levels: the IC(0) factorization order and a diagnostic
-  std::vector<int> lev(n, 0);
-  int nlev = 0;
-  for (int q = 0; q < n; ++q) {
-    const int i = lower ? q : n - 1 - q;
-    int l = 0;
-    for (int k = d.row_ptr[i]; k < d.row_ptr[i + 1]; ++k) l = std::max(l, lev[d.dep_col[k]] + 1);
-    lev[i] = l;
-    nlev = std::max(nlev, l + 1);
-  }
+  std::vector<int> lev;
+  const int nlev = row_levels(d, &lev);
   std::vector<int> order;
   {
     std::vector<int> lptr(nlev + 1, 0);
@@ -414,6 +454,7 @@ int tri_plan_build(const TriDeps& d, TriPlan* plan, int tile_rows, int level_run
 }
 
 void tri_plan_free(TriPlan* p) {
+  step_plan_free(&p->step);
   free_set(&p->r64);
   free_set(&p->r32);
   if (p->buf64s) cudaFree(p->buf64s);
@@ -505,6 +546,14 @@ int tri_default_tile_rows32(int n) {
 
 int tri_plan_fill(TriPlan* p, const double* ent_src, const double* diag_src, int mode,
                   cudaStream_t s) {
+  if (p->step.on && mode != kFillExact) {
+    GB_TRY(step_plan_fill(&p->step, ent_src, diag_src, s));
+    if (mode == kFillFma32) {
+      p->have32 = true;
+      return GB_OK;
+    }
+    mode = kFillExact;  // the exact solves' records; the FMA form is the step plan's
+  }
   const int g = std::max(1, std::min(device_sm_count() * 8, ceil_div(std::max(p->nval, p->ndiag), 256)));
   fill_records_kernel<double><<<g, 256, 0, s>>>(p->nval, p->r64.vdst, p->vsrc, ent_src, p->ndiag,
                                                 p->r64.ddst, p->r64.idst, p->dsrc, diag_src,
