@@ -243,12 +243,14 @@ int gb_debug_set_spin_budget(gb_system sys, unsigned long long ns);
 /* Test hook (host only): the lock-step solve plan of the strict lower / upper
  * part of a full CSR pattern, for values of elem_bytes (4 or 8).  tile_rows 0:
  * the planner's choice.  info: {tiles, rows of a tile, solver warps, staged
- * pages, window, inbox, most steps of a tile, pages, steps, shared bytes}.
+ * pages, own places, inbox, most steps of a tile, pages, steps, shared bytes,
+ * natural order, chunks}.
  * The arrays (NULL: sizes only): tiles [8 per tile] {row0, rows, page0, pages,
- * step0, steps, exports, 0}, ends [steps], meta [pages * 128 * 4], src
- * [pages * 128 * 4].  GB_NOT_SUPPORTED where the factor keeps its records. */
+ * step0, steps, exports, first chunk}, ends [steps], meta [pages * 128 * 4], src
+ * [pages * 128 * 4], needs [pages], thr [chunks].  GB_NOT_SUPPORTED where the factor keeps its records. */
 int gb_debug_step_plan(int n, const int *ia_host, const int *ja_host, int lower, int elem_bytes, int tile_rows,
-                       int *info, int *tiles, unsigned short *ends, unsigned *meta, int *src);
+                       int *info, int *tiles, unsigned short *ends, unsigned *meta, int *src,
+                       unsigned short *needs, unsigned short *thr);
 
 /* ------------------------------------------------------------ measurement */
 /* Per-kernel device times (ms per launch, CUDA events on the system stream)

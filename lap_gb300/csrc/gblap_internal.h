@@ -83,14 +83,19 @@ struct StepPlan {
   int ntiles = 0, tile_rows = 0;
   int nw = 0;         // solver warps
   int np = 0;         // staged pages
-  int window = 0;     // places of the tile's own values (a power of two)
+  int window = 0;     // places of the tile's own values
+  bool nat = false;   // own places in natural row order, for all the tile's rows; else a window in step order
   int nexp_max = 0;   // inbox places
   int cluster = 1, ngroups = 0;
-  int max_steps = 0;
+  int max_steps = 0, max_pages = 0;
   long long npages = 0;
   size_t smem = 0;
   void *tiles = nullptr;             // StepTile [ntiles]
   unsigned short *ends = nullptr;    // end position of each step
+  unsigned short *needs = nullptr, *thr = nullptr;  // nat: StepArgs
+  int *dsrc = nullptr;               // nat: [n] diagonal source of each row
+  void *dinv = nullptr;              // nat: [n] 1/d
+  int n = 0, lower = 0;
   unsigned char *pages = nullptr;    // [npages] row data in step order
   int *psrc = nullptr;               // [npages * kStepPage * 4] value source of each coefficient or -1
   int *pdiag = nullptr;              // [npages * kStepPage] diagonal source or -1

@@ -25,23 +25,27 @@ int upload(V** dst, const std::vector<V>& src) {
 
 size_t page_bytes(int elem) { return elem == 8 ? StepPageGeom<double>::bytes : StepPageGeom<float>::bytes; }
 
-size_t smem_bytes(int elem, int np, int window, int inbox, int max_steps) {
-  return (size_t)np * (page_bytes(elem) + (size_t)kStepPage * elem) + (size_t)(window + inbox + 2) * elem +
-         2 * (size_t)(max_steps + 3);
+size_t smem_bytes(int elem, bool nat, int np, int window, int inbox, int max_steps, int max_pages, int chunks) {
+  return (size_t)np * (page_bytes(elem) + (nat ? 0 : (size_t)kStepPage * elem)) + (size_t)(window + inbox + 2) * elem +
+         2 * (size_t)(max_steps + 4 + max_pages + chunks);
 }
-
-int threads_of(int nw) { return (nw + kStepLoaders + 2 + kStepImporters) * 32; }
 
 // The kernel a plan runs, for split-precision (FP64) or same-type right-hand sides.
 template <typename T, typename TR>
-void (*kernel_of(int k))(const StepArgs<T>, const TR*) {
-  return k <= 2 ? tri_step_kernel<T, TR, 2> : k == 3 ? tri_step_kernel<T, TR, 3> : tri_step_kernel<T, TR, 4>;
+void (*kernel_of(bool nat, int k))(const StepArgs<T>, const TR*) {
+  if (nat)
+    return k <= 2   ? tri_step_kernel<T, TR, 2, true>
+           : k == 3 ? tri_step_kernel<T, TR, 3, true>
+                    : tri_step_kernel<T, TR, 4, true>;
+  return k <= 2   ? tri_step_kernel<T, TR, 2, false>
+         : k == 3 ? tri_step_kernel<T, TR, 3, false>
+                  : tri_step_kernel<T, TR, 4, false>;
 }
 
 template <typename T, typename TR>
 int set_attributes() {
-  for (int k = 2; k <= kStepDeps; ++k) {
-    auto f = kernel_of<T, TR>(k);
+  for (int v = 0; v < 2 * (kStepDeps - 1); ++v) {
+    auto f = kernel_of<T, TR>(v & 1, 2 + v / 2);
     GB_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStepMaxSmem));
     GB_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   }
@@ -85,16 +89,20 @@ int active_clusters(K kern, int cl, int threads, size_t smem) {
 }
 
 int clusters_of(const StepPlan& p, int cl) {
-  return p.elem == 8 ? active_clusters(kernel_of<double, double>(p.k), cl, threads_of(p.nw), p.smem)
-                     : active_clusters(kernel_of<float, double>(p.k), cl, threads_of(p.nw), p.smem);
+  const int th = step_threads(p.nat, p.nw);
+  return p.elem == 8 ? active_clusters(kernel_of<double, double>(p.nat, p.k), cl, th, p.smem)
+                     : active_clusters(kernel_of<float, double>(p.nat, p.k), cl, th, p.smem);
 }
 
-// Estimated cycles of one step: the chain's own latency, and the rows' gather
-// and store, which take an L1 cycle a row each (fitted on 128^3, 64^3,
-// 97 x 61 x 83 and 1000 x 700 grids cut into tiles of 1 to 64 bands; FP64's
-// narrow pipe doubles the first).
-double step_cycles(int elem, int width) { return (elem == 8 ? 270.0 : 130.0) + 2.1 * width; }
-constexpr double kHopCycles = 150.0;      // more for a step whose inputs come from the previous tile
+// Estimated cycles of one step of a level of `width` rows, fitted on 128^3,
+// 64^3, 97 x 61 x 83 and 1000 x 700 grids cut into tiles of 1 to 44 bands
+// (FP32: 165 at 32 rows, 200 at 64, 310 at 128, 700 at 256; FP64: 320 at 16,
+// 380 at 64, 550 at 128, 1000 at 256).
+double step_cycles(int elem, int width) {
+  const double w = width;
+  return (elem == 8 ? 300.0 + 1.1 * w : 140.0 + 0.5 * w) + 0.0065 * w * w;
+}
+constexpr double kHopCycles = 250.0;      // more for a step whose inputs come from the previous tile
 constexpr double kCrossCycles = 2000.0;   // and from another cluster, through L2
 constexpr int kResidentTiles = 140;       // about what clusters of 8 to 16 place on 152 SMs
 
@@ -102,11 +110,12 @@ int warps_for(int width) { return width <= 32 ? 1 : width <= 64 ? 2 : width <= 1
 
 // The host image of a plan.
 struct StepLayout {
-  int k = 0, ntiles = 0, tile_rows = 0, nw = 0, np = 0, window = 0, nexp_max = 0, max_steps = 0;
+  int k = 0, ntiles = 0, tile_rows = 0, nw = 0, np = 0, window = 0, nexp_max = 0, max_steps = 0, max_pages = 0, max_chunks = 0;
+  bool nat = false;
   long long npages = 0;
   size_t smem = 0;
   std::vector<StepTile> tiles;
-  std::vector<unsigned short> ends;
+  std::vector<unsigned short> ends, needs, thr;
   std::vector<unsigned> meta;     // [npages * kStepPage * 4]
   std::vector<int> psrc, pdiag;
 };
@@ -210,7 +219,15 @@ bool step_layout(const TriDeps& d, const std::vector<int>& lev, int nlev, int el
       expo[i] = need[i] ? (unsigned short)ex++ : (unsigned short)kStepNone;
     }
     L->nexp_max = std::max(L->nexp_max, ex);
-    L->tiles[q] = {t0, t1 - t0, (int)L->npages, (t1 - t0 + kStepPage - 1) / kStepPage, 0, 0, ex, 0};
+    L->tiles[q] = {t0, t1 - t0, (int)L->npages, (t1 - t0 + kStepPage - 1) / kStepPage, 0, 0, ex, (int)L->thr.size()};
+    // a chunk (in the order rows are loaded) may be stored once its last row is solved
+    for (int c = 0; c < step_chunks(t1 - t0); ++c) {
+      int last = 0;
+      for (int o = c * kStepChunk; o < std::min(t1 - t0, (c + 1) * kStepChunk); ++o)
+        last = std::max(last, pos[d.lower ? t0 + o : t1 - 1 - o] + 1);
+      L->thr.push_back((unsigned short)last);
+    }
+    L->max_chunks = std::max(L->max_chunks, step_chunks(t1 - t0));
     L->npages += L->tiles[q].npages;
   }
   L->nw = warps_for(width);
@@ -228,6 +245,13 @@ bool step_layout(const TriDeps& d, const std::vector<int>& lev, int nlev, int el
       p = e;
     }
     t.nsteps = (int)L->ends.size() - t.step0;
+    int need = 0;  // chunks loaded before the rows of the pages so far may be read
+    for (int p = 0; p < t.npos; ++p) {
+      const int o = order[t.row0 + p] - t.row0;
+      need = std::max(need, (d.lower ? o : t.npos - 1 - o) / kStepChunk + 1);
+      if ((p + 1) % kStepPage == 0 || p + 1 == t.npos) L->needs.push_back((unsigned short)need);
+    }
+    L->max_pages = std::max(L->max_pages, t.npages);
     L->max_steps = std::max(L->max_steps, t.nsteps);
     // a place is written again `window` positions later: in a later step
     // than every reader's
@@ -237,13 +261,26 @@ bool step_layout(const TriDeps& d, const std::vector<int>& lev, int nlev, int el
         if (c >= t.row0 && c < t.row0 + t.npos) reach = std::max(reach, step_end[pos[i]] - pos[c]);
       }
   }
-  L->window = 32;
-  while (L->window < reach) L->window <<= 1;
-  if (L->window + L->nexp_max + 1 > 65535) return false;
-  L->np = kStepMaxPages;
-  while (L->np > 8 && smem_bytes(elem, L->np, L->window, L->nexp_max, L->max_steps) > kStepMaxSmem) L->np /= 2;
-  L->smem = smem_bytes(elem, L->np, L->window, L->nexp_max, L->max_steps);
-  if (L->smem > kStepMaxSmem) return false;
+  // The rows' own places in natural order where levels are wide and all of
+  // them fit beside the inbox: right-hand sides and solutions then move by
+  // whole lines (128^3 split lower solve 91 us, 124 in a window).  Else a
+  // window in step order, its right-hand sides gathered row by row: with one
+  // solver warp the chain is all, and the window's is shorter by an LDS and
+  // an address (1000 x 700: 161 us, 180 in natural order).
+  bool fits = false;
+  for (int form = L->nw > 1 ? 0 : 1; form < 2 && !fits; ++form) {
+    L->nat = form == 0;
+    L->window = 32;
+    if (L->nat) L->window = (R + 31) & ~31;
+    else while (L->window < reach) L->window <<= 1;
+    if (L->window + L->nexp_max + 1 > 65535) continue;
+    for (L->np = kStepMaxPages; L->np >= 8 && !fits; L->np /= 2) {
+      L->smem = smem_bytes(elem, L->nat, L->np, L->window, L->nexp_max, L->max_steps, L->max_pages, L->max_chunks);
+      fits = L->smem <= kStepMaxSmem;
+      if (fits) break;
+    }
+  }
+  if (!fits) return false;
   L->k = std::max(2, kmax);
   L->ntiles = nt;
   L->tile_rows = R;
@@ -259,14 +296,16 @@ bool step_layout(const TriDeps& d, const std::vector<int>& lev, int nlev, int el
       if (p < t.npos) {
         const int i = order[t.row0 + p];
         L->pdiag[P] = d.diag_src[i];
-        who = (unsigned)(i - t.row0) | (unsigned)expo[i] << 16;
+        who = (unsigned)(L->nat ? step_place(i - t.row0) : i - t.row0) | (unsigned)expo[i] << 16;
         int u = 0;
         for (int own = 0; own < 2; ++own)  // other tiles' terms first, each kind in column order
           for (int k = d.row_ptr[i]; k < d.row_ptr[i + 1]; ++k) {
             const int c = d.dep_col[k];
             const bool in = c >= t.row0 && c < t.row0 + t.npos;
             if (in != (own == 1)) continue;
-            place[u] = in ? (unsigned)pos[c] & (unsigned)(L->window - 1) : (unsigned)(L->window + expo[c]);
+            place[u] = !in      ? (unsigned)(L->window + expo[c])
+                       : L->nat ? (unsigned)step_place(c - t.row0)
+                                : (unsigned)pos[c] & (unsigned)(L->window - 1);
             L->psrc[P * kStepDeps + u] = d.dep_src[k];
             ++u;
           }
@@ -295,6 +334,10 @@ int step_plan_build(const TriDeps& d, const std::vector<int>& lev, int nlev, int
     plan->window = L.window;
     plan->nexp_max = L.nexp_max;
     plan->max_steps = L.max_steps;
+    plan->max_pages = L.max_pages;
+    plan->nat = L.nat;
+    plan->n = d.n;
+    plan->lower = d.lower;
     plan->npages = L.npages;
     plan->smem = L.smem;
     GB_TRY(prepare_device());
@@ -321,6 +364,12 @@ int step_plan_build(const TriDeps& d, const std::vector<int>& lev, int nlev, int
     plan->tiles = dt;
     GB_TRY(upload(&plan->ends, L.ends));
     GB_TRY(upload(&plan->psrc, L.psrc));
+    if (L.nat) {
+      GB_TRY(upload(&plan->needs, L.needs));
+      GB_TRY(upload(&plan->thr, L.thr));
+      GB_TRY(upload(&plan->dsrc, d.diag_src));
+      GB_CUDA_TRY(cudaMalloc(&plan->dinv, (size_t)d.n * elem));
+    }
     GB_TRY(upload(&plan->pdiag, L.pdiag));
     const size_t PB = page_bytes(elem);
     GB_CUDA_TRY(cudaMalloc(&plan->pages, (size_t)L.npages * PB));
@@ -331,13 +380,15 @@ int step_plan_build(const TriDeps& d, const std::vector<int>& lev, int nlev, int
     GB_CUDA_TRY(cudaMalloc(&plan->ticket, sizeof(unsigned)));
     GB_CUDA_TRY(cudaMemset(plan->ticket, 0, sizeof(unsigned)));
     plan->on = true;
+    GB_TRY(step_plan_reset(plan, 0));
+    GB_CUDA_TRY(cudaStreamSynchronize(0));
     return GB_OK;
   }
   return GB_OK;
 }
 
 void step_plan_free(StepPlan* p) {
-  void* ptrs[] = {p->tiles, p->ends, p->pages, p->psrc, p->pdiag, p->mail, p->ticket};
+  void* ptrs[] = {p->tiles, p->ends, p->pages, p->psrc, p->pdiag, p->mail, p->ticket, p->needs, p->thr, p->dsrc, p->dinv};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   *p = StepPlan();
@@ -372,6 +423,14 @@ __global__ void step_fill_kernel(long long rows, const int* __restrict__ psrc, c
   }
 }
 
+template <typename T>
+__global__ void step_dinv_kernel(int n, const int* __restrict__ dsrc, const double* __restrict__ dg, T* dinv) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double d = dg[dsrc[i]];
+    dinv[i] = (T)(d != 0.0 ? 1.0 / d : 0.0);
+  }
+}
+
 int step_plan_fill(const StepPlan* p, const double* ent, const double* dg, cudaStream_t s) {
   const long long rows = p->npages * kStepPage;
   if (rows <= 0) return GB_OK;
@@ -381,6 +440,11 @@ int step_plan_fill(const StepPlan* p, const double* ent, const double* dg, cudaS
   else
     step_fill_kernel<float><<<grid, 256, 0, s>>>(rows, p->psrc, p->pdiag, ent, dg, p->pages);
   GB_CUDA_TRY(cudaGetLastError());
+  if (p->nat) {
+    if (p->elem == 8) step_dinv_kernel<double><<<grid, 256, 0, s>>>(p->n, p->dsrc, dg, (double*)p->dinv);
+    else step_dinv_kernel<float><<<grid, 256, 0, s>>>(p->n, p->dsrc, dg, (float*)p->dinv);
+    GB_CUDA_TRY(cudaGetLastError());
+  }
   return GB_OK;
 }
 
@@ -394,9 +458,10 @@ int step_plan_reset(const StepPlan* p, cudaStream_t s) {
 template <typename T, typename TR>
 int step_solve(const StepPlan& p, const TR* rhs, T* y, const int* done, int* err, cudaStream_t s) {
   if (!p.on || p.elem != (int)sizeof(T)) return GB_NOT_SUPPORTED;
-  auto kern = kernel_of<T, TR>(p.k);
+  auto kern = kernel_of<T, TR>(p.nat, p.k);
+  const int threads = step_threads(p.nat, p.nw);
   int clusters = p.ngroups;
-  if (p.ngroups > 1) clusters = std::max(1, std::min(p.ngroups, active_clusters(kern, p.cluster, threads_of(p.nw), p.smem)));
+  if (p.ngroups > 1) clusters = std::max(1, std::min(p.ngroups, active_clusters(kern, p.cluster, threads, p.smem)));
   StepArgs<T> A;
   A.ntiles = p.ntiles;
   A.ngroups = p.ngroups;
@@ -409,6 +474,12 @@ int step_solve(const StepPlan& p, const TR* rhs, T* y, const int* done, int* err
   A.claims = (unsigned)(clusters == p.ngroups ? p.ngroups : p.ngroups + clusters);
   A.tiles = (const StepTile*)p.tiles;
   A.ends = p.ends;
+  A.needs = p.needs;
+  A.thr = p.thr;
+  A.dinv = (const T*)p.dinv;
+  A.lower = p.lower;
+  A.max_steps = p.max_steps;
+  A.max_pages = p.max_pages;
   A.pages = p.pages;
   A.mail = (T*)p.mail;
   A.ticket = p.ticket;
@@ -422,7 +493,7 @@ int step_solve(const StepPlan& p, const TR* rhs, T* y, const int* done, int* err
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3(clusters * p.cluster);
-  cfg.blockDim = dim3(threads_of(p.nw));
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = p.smem;
   cfg.stream = s;
   cfg.attrs = attr;
@@ -432,7 +503,7 @@ int step_solve(const StepPlan& p, const TR* rhs, T* y, const int* done, int* err
 }
 // The host layout for the strict one-sided part of a full CSR pattern.
 int step_layout_debug(int n, const int* ia, const int* ja, int lower, int elem, int tile_rows, int* info, int* tiles,
-                      unsigned short* ends, unsigned* meta, int* src) {
+                      unsigned short* ends, unsigned* meta, int* src, unsigned short* needs, unsigned short* thr) {
   TriDeps d;
   d.n = n;
   d.lower = lower != 0;
@@ -461,13 +532,15 @@ int step_layout_debug(int n, const int* ia, const int* ja, int lower, int elem, 
   for (int R : heights)
     if ((ok = step_layout(d, lev, nlev, elem, kmax, R, &L))) break;
   if (!ok) return GB_NOT_SUPPORTED;
-  const int v[10] = {L.ntiles, L.tile_rows, L.nw,        L.np,        L.window,
-                     L.nexp_max, L.max_steps, (int)L.npages, (int)L.ends.size(), (int)L.smem};
-  std::copy(v, v + 10, info);
+  const int v[12] = {L.ntiles, L.tile_rows, L.nw,        L.np,        L.window,
+                     L.nexp_max, L.max_steps, (int)L.npages, (int)L.ends.size(), (int)L.smem, L.nat, (int)L.thr.size()};
+  std::copy(v, v + 12, info);
   if (tiles) memcpy(tiles, L.tiles.data(), sizeof(StepTile) * L.tiles.size());
   if (ends) std::copy(L.ends.begin(), L.ends.end(), ends);
   if (meta) std::copy(L.meta.begin(), L.meta.end(), meta);
   if (src) std::copy(L.psrc.begin(), L.psrc.end(), src);
+  if (needs) std::copy(L.needs.begin(), L.needs.end(), needs);
+  if (thr) std::copy(L.thr.begin(), L.thr.end(), thr);
   return GB_OK;
 }
 
@@ -479,7 +552,8 @@ template int step_solve<double, double>(const StepPlan&, const double*, double*,
 
 extern "C" int gb_debug_step_plan(int n, const int* ia_host, const int* ja_host, int lower, int elem_bytes,
                                   int tile_rows, int* info, int* tiles, unsigned short* ends, unsigned* meta,
-                                  int* src) {
+                                  int* src, unsigned short* needs, unsigned short* thr) {
   if (n <= 0 || !ia_host || !ja_host || !info || (elem_bytes != 4 && elem_bytes != 8)) return GB_BAD_INPUT;
-  return gb::step_layout_debug(n, ia_host, ja_host, lower, elem_bytes, tile_rows, info, tiles, ends, meta, src);
+  return gb::step_layout_debug(n, ia_host, ja_host, lower, elem_bytes, tile_rows, info, tiles, ends, meta, src,
+                               needs, thr);
 }

@@ -12,30 +12,37 @@
 // per value, and a record's own ~2,500 cycles of code, not the hand-off,
 // set its pace (about 1,080 cycles a level on 128^3).  Here everything that
 // is not the chain is done by other warps beforehand, and the chain itself
-// is as short as it can be made:
+// is as short as it can be made (165 to 310 cycles a level of 32 to 128
+// rows, FP32):
 //   * a tile is solved by `nw` solver warps in lock step: one STEP is up to
 //     32*nw rows of one level, a named barrier ends it.  The barrier makes
 //     the tile's values plain shared-memory loads -- no sentinel, no poll,
-//     no counter -- and frees staged rows and value slots without further
+//     no counter -- and frees staged rows and value places without further
 //     signalling;
 //   * a row is two or three 16-byte loads from the staged page: its values'
-//     places in shared memory (resolved at plan time: the tile's own window,
-//     the inbox, or a zero), its coefficients, and its scaled right-hand
-//     side.  They are loaded one step ahead;
-//   * loader warps gather the right-hand side pages ahead and scale it, so
-//     neither the gather's latency nor FP64 conversions are on the chain;
+//     places in shared memory (resolved at plan time: its tile's own, the
+//     inbox, or a zero) and its coefficients.  They are loaded one step
+//     ahead;
 //   * the rows' static data is one stream of kStepPage-row pages in step
-//     order, copied by TMA into a ring (a barrier per page, counts of loaded pages and of solved rows);
+//     order, copied by TMA into a ring by the page warp;
+//   * right-hand sides are scaled into place by loader warps.  In natural
+//     order (NAT: wide levels) each row has its own place in shared memory,
+//     which holds its scaled right-hand side and then its value, so both
+//     move by whole lines; else a loader gathers a page's right-hand sides
+//     row by row, and solvers store their values row by row;
+//   * the stager warp counts the rows whose data is there, and the gate warp
+//     joins the solvers' barrier only once the next rows are: solver warps
+//     check nothing and branch on nothing;
 //   * a tile depends on the previous tile only.  That tile pushes the values
 //     its successor needs into the successor's inbox: through distributed
-//     shared memory inside a cluster, through a small mailbox in global
-//     memory between clusters (import warps poll it and put the sentinel
-//     back, so no output vector needs a sentinel fill).
+//     shared memory inside a cluster (~450 cycles), through a small mailbox
+//     in global memory between clusters (~1 us; import warps poll it and put
+//     the sentinel back, so no output vector needs a sentinel fill).
 //
-// Measured against the record kernel, whole solves to 1e-12: 128^3 IC(0) split
-// 189.9 -> 104.4 ms, FP64 240.2 -> 137.3 ms; 64^3 with a refactorisation
-// 130.3 -> 32.9 ms; Gauss-Seidel on 97 x 61 x 83 164.2 -> 54.3 ms (its planes
-// fit no power-of-two tile); 1000 x 700 forward + adjoint 132.0 -> 84.9 ms.
+// Measured against the record kernel, IC(0) solves (lower / upper with r'w):
+// 128^3 split 200 / 248 -> 88 / 106 us, FP64 271 / 337 -> 142 / 158 us; 64^3
+// split 243 / 245 -> 38 / 48 us; 97 x 61 x 83 207 / 253 -> 49 / 60 us (its
+// planes fit no power-of-two tile); 1000 x 700 377 / 383 -> 151 / 164 us.
 //
 // Progress: a tile depends only on the tile before it, groups of tiles are
 // claimed by ticket in order by running clusters, and every staged page's
@@ -51,17 +58,21 @@
 
 namespace gb {
 
-constexpr int kStepLoaders = 8;    // warps gathering right-hand sides
-constexpr int kStepImporters = 2;  // warps polling the mailbox of the previous cluster
-constexpr int kStepImportBatch = 8;
-constexpr int kStepMaxThreads = (kStepMaxWarps + kStepLoaders + 2 + kStepImporters) * 32;
+constexpr int kStepImportDepth = 3;  // groups of the mailbox an import warp keeps in flight
+constexpr int kStepMaxThreads = 20 * 32;
+static_assert(kStepMaxThreads >= step_threads(true, kStepMaxWarps) && kStepMaxThreads >= step_threads(false, kStepMaxWarps),
+              "the widest launch");
 
 template <typename T>
 struct StepArgs {
-  int ntiles, ngroups, nw, np, np_shift, window, inbox;
+  int ntiles, ngroups, nw, np, np_shift, window, inbox, max_steps, max_pages;
   unsigned claims;                        // ticket claims of one launch (it wraps to 0)
   const StepTile* __restrict__ tiles;     // [ntiles]
   const unsigned short* __restrict__ ends;  // steps' end positions, tile after tile
+  const unsigned short* __restrict__ needs;  // NAT: chunks loaded before a page's rows may be read
+  const unsigned short* __restrict__ thr;    // NAT: positions solved before a chunk may be stored
+  const T* __restrict__ dinv;                // NAT: 1/d, natural row order
+  int lower;
   const unsigned char* __restrict__ pages;
   T* mail;           // [ngroups][nexp_max], sentinel between launches
   unsigned* ticket;
@@ -134,10 +145,8 @@ __device__ __forceinline__ void st_global_if(bool on, double* p, double v) {
                "d"(v)
                : "memory");
 }
-__device__ __forceinline__ void sts_s32_if(bool on, uint32_t a, int v) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %0, 0;\n @p st.volatile.shared.s32 [%1], %2;\n}" ::"r"((int)on),
-               "r"(a), "r"(v)
-               : "memory");
+__device__ __forceinline__ void sts_s32(uint32_t a, int v) {
+  asm volatile("st.volatile.shared.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 // One look at a phase, without try_wait's suspension.
 __device__ __forceinline__ bool mbar_test_wait(uint64_t* b, unsigned parity) {
@@ -149,7 +158,6 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* b, unsigned parity) {
       : "memory");
   return ok != 0;
 }
-// Named barrier 1 among `threads` threads; true when any brought `bad`.
 __device__ __forceinline__ int ld_acquire_cta(uint32_t a) {
   int v;
   asm volatile("ld.acquire.cta.shared::cta.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
@@ -158,34 +166,28 @@ __device__ __forceinline__ int ld_acquire_cta(uint32_t a) {
 __device__ __forceinline__ void st_release_cta(uint32_t a, int v) {
   asm volatile("st.release.cta.shared::cta.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
-__device__ __forceinline__ bool bar_any(int threads, bool bad) {
-  int any;
-  asm volatile(
-      "{\n .reg .pred p, q;\n setp.ne.b32 p, %1, 0;\n barrier.cta.red.or.pred q, 1, %2, p;\n selp.s32 %0, 1, 0, q;\n}"
-      : "=r"(any)
-      : "r"((int)bad), "r"(threads)
-      : "memory");
-  return any != 0;
+__device__ __forceinline__ int lds_s32(uint32_t a) {
+  int v;
+  asm volatile("ld.volatile.shared.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
 }
-
-// Out of line: a value the previous tile has not pushed yet; the sentinel
-// when the wait gave up.
-template <typename T>
-__device__ __noinline__ T step_wait_value(uint32_t a, int* err) {
-  SpinClock clk;
-  for (unsigned polls = 1;; ++polls) {
-    T v;
-    lds_value(a, v);
-    if (!is_sentinel(v)) return v;
-    if ((polls & 255u) == 0u && clk.expired(err)) return v;
-  }
+// The steps' barrier, of the solver warps and the gate.  (A barrier that also
+// reduces a predicate, barrier.red, cost 90-400 cycles more a step: 1000 x
+// 700 solve 503 us against 189, 128^3 127 against 90.)
+__device__ __forceinline__ void step_barrier(int threads) {
+  asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+}
+__device__ __forceinline__ void st_release_if(bool on, uint32_t a, int v) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %0, 0;\n @p st.release.cta.shared::cta.b32 [%1], %2;\n}" ::"r"((int)on),
+               "r"(a), "r"(v)
+               : "memory");
 }
 
 // A row as the solver holds it: where its values lie, its coefficients and
 // its scaled right-hand side.
 template <typename T, int K>
 struct StepRow {
-  uint32_t at[K];
+  uint32_t at[K], own;
   T l[K];
   T acc;
   unsigned s01, s23, le;
@@ -193,17 +195,23 @@ struct StepRow {
 
 // Where a tile's staged data lies in shared memory (32-bit addresses).
 struct StepShared {
-  uint32_t ring, vals, ends, prog, loaded;
+  uint32_t ring, vals, ends, prog, staged, loaded, late;
 };
 
 // One solver warp's part of a tile.  K: the most dependencies a row has.
 // Per step and warp: the row's values (LDS), the next step's row (LDS, off
-// the chain), K FMAs, the value's store, the barrier.  The gate warp has seen
-// to the next step's pages.  False when a wait gave up.
-template <typename T, int K>
-__device__ __forceinline__ bool step_solve_tile(const StepArgs<T>& A, const StepTile& ti, unsigned base, int first,
+// the chain), K FMAs, the value's store, the barrier -- and no branch but the
+// rare wait for a value: each one costs the chain tens of cycles (a check of
+// the staged rows and a page-wise progress word here instead of in the gate:
+// 1000 x 700 solve 337 us against 189).  So nothing here fails: a value
+// waited for in vain is taken as NaN and marks the tile late, and rows that
+// were not staged in time are whatever the ring holds -- always rows of this
+// plan, whose places are in bounds; the error word is set either way.
+template <typename T, int K, bool NAT>
+__device__ __forceinline__ void step_solve_tile(const StepArgs<T>& A, const StepTile& ti, unsigned base, int first,
                                                 const StepShared& S, T* out) {
   using G = StepPageGeom<T>;
+  constexpr uint32_t kSlot = NAT ? G::bytes : G::slot;
   const unsigned npm = (unsigned)A.np - 1u;
   const unsigned wmask = (unsigned)A.window - 1u;
   const int threads = (A.nw + 1) * 32;  // solvers and gate
@@ -212,7 +220,7 @@ __device__ __forceinline__ bool step_solve_tile(const StepArgs<T>& A, const Step
   // the last one again, which is then not stored
   auto load = [&](StepRow<T, K>& r, int a, int b) {
     const unsigned p = (unsigned)min(a + first, b - 1);
-    const uint32_t pg = S.ring + ((base + (p >> kStepPageShift)) & npm) * G::slot;
+    const uint32_t pg = S.ring + ((base + (p >> kStepPageShift)) & npm) * kSlot;
     const uint32_t e = p & (kStepPage - 1);
     const uint4 m = lds128(pg + e * 16);
     const uint4 c = lds128(pg + G::coef + e * 16);
@@ -230,7 +238,7 @@ __device__ __forceinline__ bool step_solve_tile(const StepArgs<T>& A, const Step
         if constexpr (K > 3) r.l[3] = __hiloint2double((int)d.w, (int)d.z);
       }
     }
-    lds_value(pg + G::bytes + e * (uint32_t)sizeof(T), r.acc);
+    if constexpr (!NAT) lds_value(pg + G::bytes + e * (uint32_t)sizeof(T), r.acc);
     r.s01 = m.x;
     r.s23 = m.y;
     r.le = m.z;
@@ -240,27 +248,37 @@ __device__ __forceinline__ bool step_solve_tile(const StepArgs<T>& A, const Step
     r.at[1] = S.vals + (r.s01 >> 16) * (uint32_t)sizeof(T);
     if constexpr (K > 2) r.at[2] = S.vals + (r.s23 & 0xffffu) * (uint32_t)sizeof(T);
     if constexpr (K > 3) r.at[3] = S.vals + (r.s23 >> 16) * (uint32_t)sizeof(T);
+    if constexpr (NAT) r.own = S.vals + (r.le & 0xffffu) * (uint32_t)sizeof(T);
   };
   int a = 0, b = (int)lds_u16(S.ends), nb = (int)lds_u16(S.ends + 2);
   uint32_t ep = S.ends + 4;
-  // one step: solves `c`, stages the next into `n`; false when a wait gave up
-  auto step = [&](StepRow<T, K>& c, StepRow<T, K>& n) -> bool {
+  // one step: solves `c`, loads the next rows into `n`
+  auto step = [&](StepRow<T, K>& c, StepRow<T, K>& n) {
     T v[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) lds_value(c.at[k], v[k]);
+    if constexpr (NAT) lds_value(c.own, c.acc);  // the scaled rhs, until the row is solved
     const int nnb = (int)lds_u16(ep);  // the list ends in copies of the last end
     ep += 2;
     load(n, b, nb);
-    bool bad = false, miss = false;  // only the inbox's places can hold the sentinel
+    bool miss = false;  // only the inbox's places can hold the sentinel
 #pragma unroll
     for (int k = 0; k < K; ++k) miss |= is_sentinel(v[k]);
     if (miss) {
+      SpinClock clk;
+      for (unsigned polls = 1; miss; ++polls) {
+        miss = false;
 #pragma unroll
-      for (int k = 0; k < K; ++k)
-        if (is_sentinel(v[k])) {
-          v[k] = step_wait_value<T>(c.at[k], A.err);
-          bad = bad || is_sentinel(v[k]);
+        for (int k = 0; k < K; ++k)
+          if (is_sentinel(v[k])) {
+            lds_value(c.at[k], v[k]);
+            miss |= is_sentinel(v[k]);
+          }
+        if (miss && (polls & 255u) == 0u && (lds_s32(S.late) != 0 || clk.expired(A.err))) {
+          sts_s32(S.late, 1);
+          miss = false;  // the sentinel is a NaN
         }
+      }
     }
     // an FMA never returns the sentinel (a signalling NaN)
     T acc = c.acc;
@@ -269,61 +287,147 @@ __device__ __forceinline__ bool step_solve_tile(const StepArgs<T>& A, const Step
     decode(n);  // beside the FMAs: its loads are back with the values
     const int p = a + first;
     const bool on = p < b;
-    sts_value_if(on, S.vals + ((unsigned)p & wmask) * (uint32_t)sizeof(T), acc);
+    sts_value_if(on, NAT ? c.own : S.vals + ((unsigned)p & wmask) * (uint32_t)sizeof(T), acc);
     const unsigned ex = c.le >> 16;
     st_export_if(on && ex != kStepNone, out + ex, acc);
-    const bool any = bar_any(threads, bad);
-    st_global_if(on, yt + (c.le & 0xffffu), acc);
+    step_barrier(threads);
+    if constexpr (!NAT) st_global_if(on && (c.le & 0xffffu) < (unsigned)ti.npos, yt + (c.le & 0xffffu), acc);
     a = b;
     b = nb;
     nb = nnb;
-    return !any;
   };
   StepRow<T, K> r0, r1;
-  if (bar_any(threads, false)) return false;  // the first two steps' pages are there
+  step_barrier(threads);  // the first two steps' rows are staged
   load(r0, a, b);
   decode(r0);
   for (int s = 0; s < ti.nsteps; s += 2) {  // an odd count's last step is empty
-    if (!step(r0, r1)) return false;
-    if (!step(r1, r0)) return false;
+    step(r0, r1);
+    step(r1, r0);
   }
-  return true;
 }
 
-// The gate warp: waits for the pages of the rows the solvers load next, joins
-// the steps' barriers and publishes how far they are.
+// The gate warp: joins the steps' barriers, which it enters only once the
+// rows of the step after next are staged, and publishes how far the steps
+// are.  It does nothing else: with the stager's work in it it took ~340
+// cycles a step and set the pace.
 template <typename T>
 __device__ __forceinline__ bool step_gate_tile(const StepArgs<T>& A, const StepTile& ti, int lane,
                                                const StepShared& S) {
   const int threads = (A.nw + 1) * 32;
-  int avail = 0;  // pages known to be ready
-  // Loader w finishes pages (w >> 2) + k * (kStepLoaders / 4) in order and
-  // counts them: the first page one of them still owes ends what is ready.
-  auto pages = [&](int b) -> bool {
-    const int need = (b - 1) >> kStepPageShift;
-    if (need < avail) return true;
+  int staged = 0;
+  bool ok = true;
+  auto wait = [&](int end) {
     SpinClock clk;
-    for (unsigned polls = 1;; ++polls) {
-      int owed = 0x7fffffff;
-      if (lane < kStepLoaders) owed = (lane >> 2) + ld_acquire_cta(S.loaded + lane * 4) * (kStepLoaders / 4);
-      avail = (int)__reduce_min_sync(0xffffffffu, (unsigned)owed);
-      if (need < avail) return true;
-      const bool stop = (polls & 255u) == 0u && clk.expired(A.err);
-      if (__any_sync(0xffffffffu, stop)) return false;
+    for (unsigned polls = 1; ok; ++polls) {
+      staged = ld_acquire_cta(S.staged);
+      if (staged >= end) return;
+      if ((polls & 255u) == 0u && clk.expired(A.err)) ok = false;
     }
+    staged = 0x7fffffff;  // gave up: the solvers run on unguarded
   };
-  bool bad = !pages((int)lds_u16(S.ends + 2));
-  if (bar_any(threads, bad)) return false;
-  uint32_t ep = S.ends;
-  for (int s = 0; s < ((ti.nsteps + 1) & ~1); ++s, ep += 2) {
-    bad = !pages((int)lds_u16(ep + 4));
-    if (bar_any(threads, bad)) return false;
-    sts_s32_if(lane == 0, S.prog, (int)lds_u16(ep));
+  int b = (int)lds_u16(S.ends), nb = (int)lds_u16(S.ends + 2), nnb = (int)lds_u16(S.ends + 4);
+  if (nb > staged) wait(nb);
+  step_barrier(threads);
+  uint32_t at = S.ends + 6;
+  const int steps = (ti.nsteps + 1) & ~1;
+  for (int s = 0; s < steps; ++s, at += 2) {
+    if (nnb > staged) wait(nnb);
+    step_barrier(threads);
+    st_release_if(lane == 0, S.prog, b);
+    b = nb;
+    nb = nnb;
+    nnb = (int)lds_u16(at);
+  }
+  return ok;
+}
+
+// The stager warp: publishes how many rows are staged, page by page -- landed
+// (NAT; the loaders have seen to it otherwise) and with their scaled
+// right-hand sides in place.
+template <typename T, bool NAT>
+__device__ __forceinline__ bool step_stage_tile(const StepArgs<T>& A, const StepTile& ti, unsigned base, int lane,
+                                                const StepShared& S, const unsigned short* needs, uint64_t* full) {
+  constexpr int kLoaders = NAT ? kStepChunkWarps : kStepLoaders;
+  int avail = 0;  // NAT: chunks loaded; else pages with their right-hand sides
+  for (int page = 0; page < ti.npages; ++page) {
+    if constexpr (NAT) {
+      const unsigned u = base + (unsigned)page, slot = u & ((unsigned)A.np - 1u);
+      if (!__all_sync(0xffffffffu, mbar_wait(&full[slot], (u >> A.np_shift) & 1u, A.err))) return false;
+    }
+    const int need = NAT ? (int)needs[page] : page + 1;
+    if (avail < need) {  // the least of the loader warps' counts
+      SpinClock clk;
+      for (unsigned polls = 1;; ++polls) {
+        const int c = lane < kLoaders ? ld_acquire_cta(S.loaded + lane * 4) : 0x7fffffff;
+        avail = (int)__reduce_min_sync(0xffffffffu, (unsigned)c);
+        if (avail >= need) break;
+        const bool stop = (polls & 255u) == 0u && clk.expired(A.err);
+        if (__any_sync(0xffffffffu, stop)) return false;
+      }
+    }
+    if (!NAT) page = avail - 1;  // as many as they have finished
+    if (lane == 0) st_release_cta(S.staged, (page + 1) * kStepPage);
   }
   return true;
 }
 
-// One loader warp: a quarter of every (kStepLoaders / 4)-th page, in batches
+// Natural order (NAT): the rows' scaled right-hand sides go into the rows'
+// own places in row order, by whole lines; once the rows of a chunk are
+// solved the same warps write them out, by whole lines.
+template <typename T, typename TR>
+__device__ __forceinline__ bool step_stream_rows(const StepArgs<T>& A, const StepTile& ti, int lw, int lane, T* vals,
+                                                 const unsigned short* thr, const int* prog,
+                                                 const TR* __restrict__ rhs, uint32_t loaded) {
+  constexpr int kBatch = 4;
+  const int chunks = step_chunks(ti.npos);
+  const TR* const rt = rhs + ti.row0;
+  const T* const dt = A.dinv + ti.row0;
+  for (int c0 = 0; c0 < chunks; c0 += kBatch) {
+    TR r[kBatch];
+    T dv[kBatch];
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      const int o = (c0 + j) * kStepChunk + lw * 32 + lane;
+      if (c0 + j < chunks && o < ti.npos) {
+        const int i = A.lower ? o : ti.npos - 1 - o;
+        r[j] = __ldg(rt + i);
+        dv[j] = __ldg(dt + i);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      const int o = (c0 + j) * kStepChunk + lw * 32 + lane;
+      if (c0 + j < chunks && o < ti.npos) {
+        const int i = A.lower ? o : ti.npos - 1 - o;
+        vals[step_place(i)] = (T)r[j] * dv[j];
+      }
+    }
+    __syncwarp();
+    if (lane == 0) st_release_cta(loaded, min(c0 + kBatch, chunks));
+  }
+  T* const yt = A.y + ti.row0;
+  for (int c = 0; c < chunks; ++c) {
+    const int need = thr[c];
+    SpinClock clk;
+    bool ok = true;
+    for (unsigned polls = 1; ld_acquire_cta(smem_u32(prog)) < need; ++polls) {
+      if ((polls & 255u) == 0u && clk.expired(A.err)) {
+        ok = false;
+        break;
+      }
+      __nanosleep(64);
+    }
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    const int o = c * kStepChunk + lw * 32 + lane;
+    if (o < ti.npos) {
+      const int i = A.lower ? o : ti.npos - 1 - o;
+      yt[i] = vals[step_place(i)];
+    }
+  }
+  return true;
+}
+
+// One loader warp (!NAT): a quarter of every page, in batches
 // of the pages that have landed (kBatch at most): all of a batch's gathers in
 // flight together, then one release for the batch -- a release with gathers
 // outstanding waits for them (one page at a time: ~450 cycles a page).
@@ -332,18 +436,18 @@ __device__ __forceinline__ bool step_load_rhs(const StepArgs<T>& A, const StepTi
                                               unsigned char* ring, const TR* __restrict__ rhs, uint64_t* full,
                                               uint32_t loaded) {
   using G = StepPageGeom<T>;
-  constexpr int kBatch = 4, kStride = kStepLoaders / 4;
+  static_assert(kStepLoaders * 32 == kStepPage, "a loader warp takes a quarter of each page");
+  constexpr int kBatch = 4;
   const unsigned npm = (unsigned)A.np - 1u;
-  const int e = (lw & 3) * 32 + lane;
+  const int e = lw * 32 + lane;
   const TR* const rt = rhs + ti.row0;
-  int count = 0;  // pages finished
-  for (int pg = lw >> 2; pg < ti.npages;) {
+  for (int pg = 0; pg < ti.npages;) {
     TR r[kBatch];
     T dv[kBatch];
     bool in[kBatch];
 #pragma unroll
     for (int j = 0; j < kBatch; ++j) {
-      const int p = pg + j * kStride;
+      const int p = pg + j;
       const unsigned u = base + (unsigned)p, slot = u & npm, par = (u >> A.np_shift) & 1u;
       in[j] = p < ti.npages && (j == 0 || in[j > 0 ? j - 1 : 0]);
       if (in[j]) {
@@ -368,11 +472,10 @@ __device__ __forceinline__ bool step_load_rhs(const StepArgs<T>& A, const StepTi
       if (in[j]) {
         const unsigned slot = (base + (unsigned)pg) & npm;
         reinterpret_cast<T*>(ring + slot * G::slot + G::bytes)[e] = (T)r[j] * dv[j];
-        pg += kStride;
-        ++count;
+        ++pg;
       }
     __syncwarp();
-    if (lane == 0) st_release_cta(loaded, count);
+    if (lane == 0) st_release_cta(loaded, pg);
   }
   return true;
 }
@@ -391,16 +494,21 @@ __device__ __forceinline__ bool step_wait_rows(const int* prog, int rows, int* e
 }
 
 // rhs: the right-hand side (TR; rounded to T), natural row order.
-template <typename T, typename TR, int K>
+template <typename T, typename TR, int K, bool NAT>
 __global__ void __launch_bounds__(kStepMaxThreads, 1) tri_step_kernel(const StepArgs<T> A, const TR* __restrict__ rhs) {
   using G = StepPageGeom<T>;
   extern __shared__ __align__(128) unsigned char step_smem[];
-  unsigned char* ring = step_smem;                                        // np pages, each with its scaled rhs
-  T* vals = reinterpret_cast<T*>(step_smem + (size_t)A.np * G::slot);      // window | inbox | zero
+  constexpr uint32_t kSlot = NAT ? G::bytes : G::slot;
+  constexpr int kLoaders = NAT ? kStepChunkWarps : kStepLoaders;
+  unsigned char* ring = step_smem;                                     // np pages (!NAT: with their scaled rhs)
+  T* vals = reinterpret_cast<T*>(step_smem + (size_t)A.np * kSlot);     // own places | inbox | zero
   unsigned short* ends = reinterpret_cast<unsigned short*>(vals + A.window + A.inbox + 2);
+  unsigned short* needs = ends + A.max_steps + 4;                       // NAT
+  unsigned short* thr = needs + A.max_pages;                            // NAT
   __shared__ __align__(8) uint64_t full[kStepMaxPages];
-  __shared__ int s_loaded[kStepLoaders];  // pages of the current tile each loader warp has finished
-  __shared__ int s_prog;  // rows of the current tile solved
+  __shared__ int s_loaded[kLoaders];  // pages of the current tile each loader warp has finished
+  __shared__ int s_late;  // a value of the current tile was waited for in vain
+  __shared__ int s_prog, s_staged;  // rows of the current tile solved, and staged
   __shared__ unsigned s_issued[kStepMaxPages];  // last stream page copied into each slot
   __shared__ int s_group;
   if (*A.done != 0) return;  // the whole grid: nothing writes it meanwhile
@@ -414,7 +522,9 @@ __global__ void __launch_bounds__(kStepMaxThreads, 1) tri_step_kernel(const Step
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     vals[A.window + A.inbox] = T(0);
   }
-  const int prod = A.nw + kStepLoaders, import0 = prod + 2;
+  // rows that are never staged (a timeout) must still be in bounds
+  for (unsigned i = threadIdx.x; i < A.np * kSlot / 16u; i += blockDim.x) reinterpret_cast<uint4*>(ring)[i] = make_uint4(0, 0, 0, 0);
+  const int prod = A.nw + kLoaders, import0 = prod + 3;
   unsigned base = 0;  // pages of earlier tiles streamed by this CTA
   bool failed = false;
   for (bool first = true;; first = false) {
@@ -431,21 +541,28 @@ __global__ void __launch_bounds__(kStepMaxThreads, 1) tri_step_kernel(const Step
     const int q = g * (int)cl + (int)rank;
     if (q < A.ntiles) {
       const StepTile ti = A.tiles[q];
-      for (int i = threadIdx.x; i < ti.nsteps + 3; i += blockDim.x)
+      for (int i = threadIdx.x; i < ti.nsteps + 4; i += blockDim.x)
         ends[i] = A.ends[ti.step0 + min(i, ti.nsteps - 1)];
-      if (threadIdx.x < kStepLoaders) s_loaded[threadIdx.x] = 0;
-      if (threadIdx.x == 0) s_prog = 0;
+      if constexpr (NAT) {
+        for (int i = threadIdx.x; i < ti.npages; i += blockDim.x) needs[i] = A.needs[ti.page0 + i];
+        for (int i = threadIdx.x; i < step_chunks(ti.npos); i += blockDim.x) thr[i] = A.thr[ti.thr0 + i];
+      }
+      if (threadIdx.x < kLoaders) s_loaded[threadIdx.x] = 0;
+      if (threadIdx.x == 0) s_prog = s_staged = s_late = 0;
       // where the next tile expects this one's exports
       T* out = rank + 1 < cl ? cluster_ptr(vals + A.window, q + 1 < A.ntiles ? rank + 1 : rank)
                              : A.mail + (size_t)g * A.inbox;
-      const StepShared S{smem_u32(ring), smem_u32(vals), smem_u32(ends), smem_u32(&s_prog), smem_u32(s_loaded)};
+      const StepShared S{smem_u32(ring), smem_u32(vals), smem_u32(ends), smem_u32(&s_prog), smem_u32(&s_staged),
+                         smem_u32(s_loaded), smem_u32(&s_late)};
       __syncthreads();
       if (wid < A.nw) {
-        if (!failed)
-          failed = !step_solve_tile<T, K>(A, ti, base, (int)threadIdx.x, S, out);
+        step_solve_tile<T, K, NAT>(A, ti, base, (int)threadIdx.x, S, out);
       } else if (wid < prod) {
-        failed = !step_load_rhs<T, TR>(A, ti, base, wid - A.nw, lane, ring, rhs, full,
-                                        smem_u32(s_loaded + (wid - A.nw)));
+        const uint32_t count = smem_u32(s_loaded + (wid - A.nw));
+        if constexpr (NAT)
+          failed = !step_stream_rows<T, TR>(A, ti, wid - A.nw, lane, vals, thr, &s_prog, rhs, count);
+        else
+          failed = !step_load_rhs<T, TR>(A, ti, base, wid - A.nw, lane, ring, rhs, full, count);
       } else if (wid == prod) {
         // one lane, in page order: lanes of one warp waiting on different
         // barriers would hold each other up (a try_wait suspends the warp)
@@ -459,7 +576,7 @@ __global__ void __launch_bounds__(kStepMaxThreads, 1) tri_step_kernel(const Step
               break;
             }
             mbar_expect_tx(&full[slot], G::bytes);
-            tma_load_1d(ring + slot * G::slot, src + (size_t)pg * G::bytes, G::bytes, &full[slot]);
+            tma_load_1d(ring + slot * kSlot, src + (size_t)pg * G::bytes, G::bytes, &full[slot]);
             s_issued[slot] = u;
             // L2 ahead of the ring: the stream is read once per launch
             if (pg + A.np < ti.npages) tma_prefetch_l2(src + (size_t)(pg + A.np) * G::bytes, G::bytes);
@@ -467,33 +584,43 @@ __global__ void __launch_bounds__(kStepMaxThreads, 1) tri_step_kernel(const Step
         }
         __syncwarp();
       } else if (wid == prod + 1) {
-        if (!failed) failed = !step_gate_tile<T>(A, ti, lane, S);
+        failed = !step_gate_tile<T>(A, ti, lane, S) || failed;
+      } else if (wid == prod + 2) {
+        if (!failed) failed = !step_stage_tile<T, NAT>(A, ti, base, lane, S, needs, full);
       } else if (rank == 0 && g > 0) {
         // the previous cluster's last tile: its exports, in its step order
-        const T* mail = A.mail + (size_t)(g - 1) * A.inbox;
+        T* mail = A.mail + (size_t)(g - 1) * A.inbox;
         const int cnt = A.tiles[q - 1].nexp;
-        constexpr int kLane = kStepImporters * 32;
-        for (int i0 = (wid - import0) * 32 + lane; i0 < cnt && !failed; i0 += kLane * kStepImportBatch) {
-          unsigned pend = 0;
+        // A warp takes every kWarps-th group of 32 and keeps kDepth groups'
+        // loads in flight; what has arrived goes into the inbox at once, and
+        // the warp moves on past the leading groups that are complete.
+        // (Per-lane places with their own polls ran into one L2 round trip a
+        // place: 4-5 us behind, against ~1.)
+        constexpr int kWarps = step_importers(NAT), kDepth = kStepImportDepth;
+        SpinClock clk;
+        int grp = wid - import0;
+        for (unsigned polls = 1; grp * 32 < cnt; ++polls) {
+          T v[kDepth];
 #pragma unroll
-          for (int j = 0; j < kStepImportBatch; ++j) pend |= i0 + j * kLane < cnt ? 1u << j : 0u;
-          SpinClock clk;
-          for (unsigned polls = 1; pend; ++polls) {
-            T v[kStepImportBatch];
+          for (int j = 0; j < kDepth; ++j)
+            v[j] = ld_relaxed(mail + min((grp + j * kWarps) * 32 + lane, cnt - 1));
+          int lead = 0;
 #pragma unroll
-            for (int j = 0; j < kStepImportBatch; ++j)
-              if (pend >> j & 1u) v[j] = ld_relaxed(mail + i0 + j * kLane);
-#pragma unroll
-            for (int j = 0; j < kStepImportBatch; ++j)
-              if ((pend >> j & 1u) && !is_sentinel(v[j])) {
-                *(volatile T*)(vals + A.window + i0 + j * kLane) = v[j];
-                st_relaxed(const_cast<T*>(mail) + i0 + j * kLane, sentinel<T>());
-                pend &= ~(1u << j);
-              }
-            if (pend && (polls & 63u) == 0u && clk.expired(A.err)) {
-              failed = true;
-              break;
+          for (int j = 0; j < kDepth; ++j) {
+            const int at = (grp + j * kWarps) * 32 + lane;
+            const bool here = !is_sentinel(v[j]);
+            sts_value_if(here && at < cnt, smem_u32(vals + A.window) + (uint32_t)at * (uint32_t)sizeof(T), v[j]);
+            const bool all = __all_sync(0xffffffffu, here);
+            if (lead == j && all) {
+              if (at < cnt) st_relaxed(mail + at, sentinel<T>());
+              ++lead;
             }
+          }
+          grp += lead * kWarps;
+          if (lead) clk = SpinClock();
+          else if ((polls & 63u) == 0u && __any_sync(0xffffffffu, clk.expired(A.err))) {
+            failed = true;
+            break;
           }
         }
         __syncwarp();

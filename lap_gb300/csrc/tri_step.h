@@ -12,6 +12,9 @@ constexpr int kStepPageShift = 7;
 constexpr int kStepPage = 1 << kStepPageShift;  // rows of a staged page
 constexpr int kStepMaxPages = 32;     // staged pages, at most
 constexpr int kStepMaxWarps = 8;      // solver warps, at most
+constexpr int kStepLoaders = 4;      // warps gathering right-hand sides by page
+constexpr int kStepChunkWarps = 6;   // warps streaming rows in natural order
+constexpr int kStepChunk = 32 * kStepChunkWarps;  // rows of one of their passes
 constexpr unsigned kStepNone = 0xffffu;  // a row no later tile needs
 
 // One page of kStepPage rows: per row {place 0 | place 1 << 16, place 2 |
@@ -38,13 +41,24 @@ struct StepPageGeom<double> {
   static constexpr int slot = bytes + kStepPage * 8;
 };
 
+// warps polling the mailbox of the previous cluster
+__host__ __device__ constexpr int step_importers(bool nat) { return nat ? 3 : 4; }
+// threads of a launch: solvers, loaders, page warp, gate, stager, importers
+constexpr int step_threads(bool nat, int nw) {
+  return (nw + (nat ? kStepChunkWarps : kStepLoaders) + 3 + step_importers(nat)) * 32;
+}
+__host__ __device__ inline int step_chunks(int rows) { return (rows + kStepChunk - 1) / kStepChunk; }
+// A row's own place in natural order: lines skewed by three banks each, since
+// a level of a grid walks its rows with a stride of one line less one.
+__host__ __device__ inline int step_place(int i) { return (i & ~31) | ((i + 3 * (i >> 5)) & 31); }
+
 struct StepTile {
   int row0;    // first row of the tile
   int npos;    // its rows
   int page0, npages;
   int step0, nsteps;
   int nexp;    // rows the next tile depends on
-  int pad;
+  int thr0;    // first of its chunks' thresholds
 };
 
 // Builds the plan for values of `elem` bytes where the factor allows it

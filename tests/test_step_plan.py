@@ -15,47 +15,61 @@ import pytest
 import lap_gb300 as gb
 from lap_gb300 import gen
 
-PAGE = 128
+PAGE, CHUNK = 128, 192
 
 
 def plan(A, lower, elem, tile_rows=0):
     L = gb.lib()
     ia, ja = np.ascontiguousarray(A.ia, np.int32), np.ascontiguousarray(A.ja, np.int32)
-    info = np.zeros(10, np.int32)
+    info = np.zeros(12, np.int32)
     head = (A.n, ia.ctypes.data, ja.ctypes.data, int(lower), elem, tile_rows, info.ctypes.data)
-    rc = L.gb_debug_step_plan(*head, None, None, None, None)
+    rc = L.gb_debug_step_plan(*head, *[None] * 6)
     if rc:
         return rc
     tiles = np.zeros((info[0], 8), np.int32)
     ends = np.zeros(info[8], np.uint16)
     meta = np.zeros((info[7] * PAGE, 4), np.uint32)
     src = np.zeros((info[7] * PAGE, 4), np.int32)
-    assert L.gb_debug_step_plan(*head, tiles.ctypes.data, ends.ctypes.data, meta.ctypes.data, src.ctypes.data) == 0
-    keys = ("tiles", "rows", "nw", "np", "window", "inbox", "max_steps", "pages", "steps", "smem")
-    return dict(zip(keys, (int(v) for v in info))), tiles, ends, meta, src
+    needs, thr = np.zeros(info[7], np.uint16), np.zeros(info[11], np.uint16)
+    out = (tiles, ends, meta, src, needs, thr)
+    assert L.gb_debug_step_plan(*head, *(v.ctypes.data for v in out)) == 0
+    keys = ("tiles", "rows", "nw", "np", "window", "inbox", "max_steps", "pages", "steps", "smem", "nat", "chunks")
+    return dict(zip(keys, (int(v) for v in info))), *out
 
 
 def replay(A, lower, elem, tile_rows=0):
-    info, tiles, ends, meta, src = plan(A, lower, elem, tile_rows)
-    window, inbox = info["window"], info["inbox"]
-    assert window & (window - 1) == 0 and window + inbox + 1 <= 65535
+    info, tiles, ends, meta, src, needs, thr = plan(A, lower, elem, tile_rows)
+    window, inbox, nat = info["window"], info["inbox"], info["nat"]
+    assert (nat or window & (window - 1) == 0) and window + inbox + 1 <= 65535
     assert info["smem"] <= 231168 and info["np"] in (8, 16, 32) and info["max_steps"] == tiles[:, 5].max()
     rows_of = np.repeat(np.arange(A.n), np.diff(A.ia))
     solved = np.zeros(A.n, int)
     used = np.zeros(A.nnz, int)
     before = np.full(inbox, -1)  # what the previous tile pushed: row by inbox place
     for q in range(info["tiles"]):
-        row0, npos, page0, npages, step0, nsteps, nexp, _ = tiles[q]
+        row0, npos, page0, npages, step0, nsteps, nexp, thr0 = tiles[q]
         assert 0 < npos <= npages * PAGE and nexp <= inbox
         held = np.concatenate([np.full(window, -1), before, [-2]])
         pushed = np.full(inbox, -1)
+        # natural order: where a row lies, which chunk it is loaded and stored in
+        i = np.arange(npos)
+        place_of = (i & ~31) | ((i + 3 * (i >> 5)) & 31)
+        chunk_of = (i if lower else npos - 1 - i) // CHUNK
+        if nat:
+            assert len(np.unique(place_of)) == npos and place_of.max() < window
+        at = np.zeros(npos, int)  # position of each row
         a = 0
         for s in range(step0, step0 + nsteps):
             b = int(ends[s])
             assert a < b <= min(npos, a + 32 * info["nw"])
             P = page0 * PAGE + np.arange(a, b)
             place = np.stack([meta[P, 0] & 0xffff, meta[P, 0] >> 16, meta[P, 1] & 0xffff, meta[P, 1] >> 16], 1)
-            row = row0 + (meta[P, 2] & 0xffff).astype(int)
+            own = (meta[P, 2] & 0xffff).astype(int)
+            row = row0 + (np.argsort(place_of)[np.searchsorted(np.sort(place_of), own)] if nat else own)
+            at[row - row0] = np.arange(a, b)
+            if nat:
+                assert (place_of[row - row0] == own).all()
+                assert (needs[page0 + np.arange(a, b) // PAGE] > chunk_of[row - row0]).all()
             assert place.max() <= window + inbox
             got = held[place]
             for k in range(4):
@@ -65,8 +79,9 @@ def replay(A, lower, elem, tile_rows=0):
                 assert (got[~there, k] == -2).all()  # no entry: the zero place
                 used[src[P, k][there]] += 1
             # no place read in a step is written in it: its warps are not ordered
-            assert not np.isin(np.arange(a, b) & (window - 1), place[place < window]).any()
-            held[np.arange(a, b) & (window - 1)] = row
+            written = own if nat else np.arange(a, b) & (window - 1)
+            assert not np.isin(written, place[place < window]).any()
+            held[written] = row
             ex = (meta[P, 2] >> 16).astype(int)
             out = ex != 0xffff
             assert (ex[out] < nexp).all()
@@ -74,6 +89,8 @@ def replay(A, lower, elem, tile_rows=0):
             solved[row] += 1
             a = b
         assert a == npos and (pushed[:nexp] >= 0).all()
+        for c in range(chunk_of.max() + 1 if nat else 0):
+            assert thr[thr0 + c] == at[chunk_of == c].max() + 1
         before = pushed
     assert (solved == 1).all()
     want = A.ja < rows_of if lower else A.ja > rows_of
