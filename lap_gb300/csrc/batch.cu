@@ -42,6 +42,7 @@
 #include "pcg.h"
 #include "pcg_state.cuh"
 #include "system.h"
+#include "team.h"
 
 namespace gb {
 
@@ -925,6 +926,9 @@ struct gb_batch_s {
   int rpb = kBundleRows;       // rows per SpMV bundle
   int chunk_rows = kChunkRows; // rows per update / reduction chunk
   size_t part_b_cap = 0, part_c_cap = 0;
+  TeamPlan team;       // block-diagonal: every system's loop in one launch, where they fit
+  bool no_team = false;  // the autotuner times the bundle loop
+  int* err = nullptr;  // [4] error word and spin budget of the team loop's waits
 };
 
 namespace {
@@ -953,6 +957,7 @@ void batch_free(gb_batch bt) {
     if (lg.exec) cudaGraphExecDestroy(lg.exec);
     if (lg.graph) cudaGraphDestroy(lg.graph);
   }
+  team_plan_free(&bt->team);
   for (void* v : bt->owned) cudaFree(v);
   if (bt->st_h) cudaFreeHost(bt->st_h);
   if (bt->ev0) cudaEventDestroy(bt->ev0);
@@ -1156,6 +1161,13 @@ int batch_body(gb_batch bt, int split, int maxit, cudaGraphConditionalHandle con
 
 // The iteration loop as one graph: a while node around batch_body.
 int batch_loop(gb_batch bt, int split, int maxit, int use_graph) {
+  if (bt->team.on && !bt->no_team) {
+    TeamData<double, double> d{bt->ia, bt->ja, bt->a, bt->jacobi ? bt->d_r : nullptr, bt->x, bt->r, bt->w, bt->p, bt->q,
+                               bt->row_off, bt->N, bt->st, nullptr, 0, bt->err};
+    if (!split) return team_loop(bt->team, d, bt->s);
+    TeamData<double, float> f{d.ia, d.ja, bt->a32, d.d_r, d.x, d.r, d.w, d.p, d.q, d.row_off, d.n, d.st, nullptr, 0, d.err};
+    return team_loop(bt->team, f, bt->s);
+  }
   GB_CUDA_TRY(cudaMemsetAsync(bt->tk, 0, sizeof(unsigned) * 4, bt->s));
   GB_CUDA_TRY(cudaMemsetAsync(bt->nactive, 0, sizeof(int) * 4, bt->s));
   if (!use_graph) {
@@ -1231,6 +1243,7 @@ int batch_solve(gb_batch bt, const double* b, double* x, const gb_pcg_opts* opts
   }
   GB_CUDA_TRY(cudaMemcpyAsync(bt->st, hs, sizeof(PcgState) * bt->count, cudaMemcpyHostToDevice, bt->s));
   GB_CUDA_TRY(cudaMemcpyAsync(bt->so, hs + bt->count, sizeof(PcgState) * bt->count, cudaMemcpyHostToDevice, bt->s));
+  if (bt->err) GB_CUDA_TRY(cudaMemsetAsync(bt->err, 0, sizeof(int), bt->s));
   GB_CUDA_TRY(cudaEventRecord(bt->ev0, bt->s));
   const int gt = std::max(1, std::min(ceil_div(bt->n1, kTrRows), 8 * device_sm_count()));
   if (bt->inter) {
@@ -1301,8 +1314,13 @@ int batch_solve(gb_batch bt, const double* b, double* x, const gb_pcg_opts* opts
   float ms = 0.f;
   cudaEventElapsedTime(&ms, bt->ev0, bt->ev1);
   r.device_ms = ms;
+  if (bt->err) {
+    int err = 0;
+    GB_CUDA_TRY(cudaMemcpy(&err, bt->err, sizeof(int), cudaMemcpyDeviceToHost));
+    if (err) r.status = err;
+  }
   if (res) *res = r;
-  return GB_OK;
+  return r.status == GB_TIMEOUT ? GB_TIMEOUT : GB_OK;
 }
 
 }  // namespace
@@ -1363,6 +1381,9 @@ extern "C" int gb_batch_create(int count, const long long* row_off_host, const l
   if (cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, bt->s) != cudaSuccess ||
       cudaStreamSynchronize(bt->s) != cudaSuccess)
     return fail(GB_CUDA_ERROR);
+  if ((rc = balloc(bt, &bt->err, 4)) != GB_OK) return fail(rc);
+  if (cudaMemset(bt->err, 0, sizeof(int) * 4) != cudaSuccess) return fail(GB_CUDA_ERROR);
+  if ((rc = team_plan_build(count, bt->h_roff, bt->h_ia.data(), &bt->team)) != GB_OK) return fail(rc);
   if (hbad) return fail(GB_BAD_INPUT);  // a row without a (nonzero) diagonal
   *out = bt;
   return GB_OK;
@@ -1551,10 +1572,15 @@ int batch_time(gb_batch bt, const double* b, double* x, int iters, double* ms) {
   o.tol = 0.0;
   o.maxit = iters;
   gb_pcg_result r;
-  for (int k = 0; k < 2; ++k) {
-    GB_CUDA_TRY(cudaMemsetAsync(x, 0, sizeof(double) * (size_t)bt->N, bt->s));
-    GB_TRY(batch_solve(bt, b, x, &o, nullptr, nullptr, &r));
+  bt->no_team = true;
+  int rc = GB_OK;
+  for (int k = 0; k < 2 && rc == GB_OK; ++k) {
+    rc = cudaMemsetAsync(x, 0, sizeof(double) * (size_t)bt->N, bt->s) == cudaSuccess
+             ? batch_solve(bt, b, x, &o, nullptr, nullptr, &r)
+             : GB_CUDA_ERROR;
   }
+  bt->no_team = false;
+  GB_TRY(rc);
   *ms = r.device_ms;
   return GB_OK;
 }

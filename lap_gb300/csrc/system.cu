@@ -143,6 +143,7 @@ static void system_free(gb_system s) {
   batch_release(s->multi_tail);
   s->multi_tail = nullptr;
   spmv_plan_free(&s->plan);
+  team_plan_free(&s->team);
   tri_plan_free(&s->L);
   tri_plan_free(&s->U);
   tri_plan_free(&s->L32);
@@ -289,6 +290,7 @@ extern "C" int gb_system_create(int n, int nnz, const int* ia, const int* ja, co
   CKC(cudaMemset(s->err, 0, sizeof(int) * 4));
   const int* hia = s->h_ia.data();
   const int* hja = s->h_ja.data();
+  if (prec == GB_PREC_LINE_JACOBI || prec == GB_PREC_NONE) CK(team_plan_build(1, {0, n}, hia, &s->team));
   std::vector<int> tpos;
   CK(transpose_positions(n, hia, hja, &tpos));  // also proves the pattern symmetric
   ph.mark("spmv plan + transpose");
@@ -597,6 +599,19 @@ static int run_recurrence_split(gb_system s, double tol, int maxit, const double
 
 // Runs (or resumes) the iteration loop until the recurrence's done flag.
 static int run_loop(gb_system s, int idx, BodyFn body_fn, int maxit, int use_graph) {
+  if (s->team.on && idx < 2) {  // one launch, captured or not
+    const bool jac = s->prec == GB_PREC_LINE_JACOBI;
+    if (idx == 0) {
+      auto& v = s->v64;
+      TeamData<double, double> d{s->ia, s->ja, s->a,    jac ? s->d_r : nullptr, v.x, v.r, jac ? v.w : v.r, v.p0, v.q,
+                                 nullptr, s->n, s->st, s->hist, 1, s->err};
+      return team_loop(s->team, d, s->s);
+    }
+    auto& v = s->v32;
+    TeamData<float, float> d{s->ia, s->ja, s->a32,  jac ? s->d_r32 : nullptr, v.x, v.r, jac ? v.w : v.r, v.p0, v.q,
+                             nullptr, s->n, s->st, s->hist, 1, s->err};
+    return team_loop(s->team, d, s->s);
+  }
   if (use_graph) {
     LoopGraph* lg = nullptr;
     GB_TRY(get_loop_graph(s, idx, body_fn, &lg));

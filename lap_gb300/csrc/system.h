@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "gblap_internal.h"
+#include "team.h"
 
 namespace gb {
 
@@ -94,6 +95,7 @@ struct gb_system_s {
   int pl_nnz = 0, pu_nnz = 0;                // their entry counts
   double *pv_l = nullptr, *pv_u = nullptr;   // GS_std: la / ua scattered onto A's pattern
   unsigned long long* hash_dev = nullptr;    // 8 bytes of scratch for pattern_hash
+  gb::TeamPlan team;      // line_jacobi / none: the whole recurrence in one launch, where it fits
   gb::LoopGraph loop[3];  // [precision]
   int loop_key[3] = {-1, -1, -1};
 };

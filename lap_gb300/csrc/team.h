@@ -1,0 +1,56 @@
+// team.h -- whole PCG recurrences (line_jacobi, none) in one launch
+// (team.cu has the kernel and its reasons).
+#pragma once
+
+#include <vector>
+
+#include "gblap_internal.h"
+
+namespace gb {
+
+struct PcgState;
+
+// Blocks of one launch, by system: blocks [cta0[s], cta0[s+1]) hold system
+// s's rows, kTeamThreads * rows of them each.
+struct TeamPlan {
+  bool on = false;
+  int ctas = 0, rows = 0;   // blocks; rows of a thread (1 to 4)
+  size_t smem = 0;          // bytes of matrix entries kept in shared memory (0: none)
+  int max_nnz = 0;          // most entries of a block
+  int *cta_sys = nullptr, *cta0 = nullptr;  // device [ctas], [systems + 1]
+  double *mail = nullptr;        // device: per system [blocks][4][blocks][2]
+  long long *mail0 = nullptr;    // device [systems]
+  long long mail_len = 0;
+};
+
+constexpr int kTeamThreads = 256;
+constexpr int kTeamMaxRow = 64;  // entries of a row (a thread sums its rows alone)
+
+// Plans `count` systems of rows [row_off[s], row_off[s+1]) with global row
+// pointers ia (host); plan->on says whether all their blocks fit the device
+// at once and no row is too long.
+int team_plan_build(int count, const std::vector<int>& row_off, const int* ia, TeamPlan* plan);
+void team_plan_free(TeamPlan* plan);
+
+// Vectors and matrix of the systems, concatenated; columns local to the
+// system.  d_r null: no preconditioner (w is r).
+template <typename T, typename TA>
+struct TeamData {
+  const int *ia, *ja;
+  const TA* a;
+  const T* d_r;
+  T *x, *r, *w, *p, *q;
+  const int* row_off;  // null: one system from row 0
+  int n;               // rows in all
+  PcgState* st;        // [systems]
+  double* hist;        // one system: residual history (st->hist_len entries), or null
+  int roll_done;       // rho rolls in the last iteration too (the single-system recurrence's convention)
+  int* err;
+};
+
+// Runs every system's recurrence from its state until it is done (or its
+// state says it is), as the loops of update / spmv_pq kernels do.
+template <typename T, typename TA>
+int team_loop(const TeamPlan& plan, const TeamData<T, TA>& d, cudaStream_t s);
+
+}  // namespace gb
