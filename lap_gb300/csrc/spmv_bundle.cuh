@@ -6,6 +6,8 @@
 // the products (alpha*a_j)*x(ja_j) (EXACT) or just the gathered x(ja_j) in
 // shared memory.  Phase 2: lane l sums row l's entries in column order.
 //
+// UNIT: alpha is 1, so its product with an entry is the entry.
+//
 // EXACT reproduces LAP's simple_csr_matvec (simple_blas.c:24-44) bit for
 // bit: y = beta*y, then y += (alpha*a_j)*x_j left to right with separate
 // round-to-nearest multiply and add (the reference's gcc build does not
@@ -93,7 +95,7 @@ __device__ __forceinline__ BundleHead bundle_head(int b, int n, const int* __res
   return h;
 }
 
-template <typename T, bool EXACT, typename XF, typename EP>
+template <typename T, bool EXACT, bool UNIT, typename XF, typename EP>
 __device__ __forceinline__ void spmv_bundle_h(const BundleHead& h, const int* __restrict__ ia,
                                               const int* __restrict__ ja, const T* __restrict__ a, T alpha, XF& xf,
                                               EP& ep, T* stage) {
@@ -116,7 +118,7 @@ __device__ __forceinline__ void spmv_bundle_h(const BundleHead& h, const int* __
       T s = T(0);
       for (int j = k0 + lane; j < k1; j += 32) {
         const T xv = xf(__ldg(ja + j));
-        s = EXACT ? add_rn(s, mul_rn(mul_rn(alpha, __ldg(a + j)), xv)) : fma_rn(__ldg(a + j), xv, s);
+        s = EXACT ? add_rn(s, mul_rn(UNIT ? __ldg(a + j) : mul_rn(alpha, __ldg(a + j)), xv)) : fma_rn(__ldg(a + j), xv, s);
       }
       s = warp_sum(s);
       if (lane == 0) {
@@ -130,9 +132,14 @@ __device__ __forceinline__ void spmv_bundle_h(const BundleHead& h, const int* __
 #if GB_SPMV_SHORT_ROWS
   // Every row of the bundle has at most kSpmvHeld entries (stencils): each
   // lane loads its own row's columns and values and gathers its x values,
-  // all of them in flight at once -- no staging pass.  The same FMA chain,
+  // all of them in flight at once -- no staging pass.  The same operations,
   // in the same order, as the staged form below.
-  if (!EXACT && __all_sync(0xffffffffu, !own || re - rs <= kSpmvHeld)) {
+  if ((!EXACT || UNIT) && __all_sync(0xffffffffu, !own || re - rs <= kSpmvHeld)) {
+    // EXACT skips the entries past the bundle's longest row for the whole
+    // warp: an FP64 instruction takes its pipe's 64 cycles even when every
+    // lane is predicated off.  (In the fused kernels that costs more in
+    // spills than it saves: FP64 spmv_pq 61.8 -> 66.1 us on 128^3.)
+    const int longest = EXACT ? (int)__reduce_max_sync(0xffffffffu, own ? (unsigned)(re - rs) : 0u) : kSpmvHeld;
     if (own) {
       T acc = ep.init(r);
       int c[kSpmvHeld];
@@ -146,8 +153,10 @@ __device__ __forceinline__ void spmv_bundle_h(const BundleHead& h, const int* __
 #pragma unroll
       for (int u = 0; u < kSpmvHeld; ++u) xv[u] = c[u] >= 0 ? xf(c[u]) : T(0);
 #pragma unroll
-      for (int u = 0; u < kSpmvHeld; ++u)
-        if (c[u] >= 0) acc = fma_rn(av[u], xv[u], acc);
+      for (int u = 0; u < kSpmvHeld; ++u) {
+        if (EXACT && u >= longest) break;
+        if (c[u] >= 0) acc = EXACT ? add_rn(acc, mul_rn(av[u], xv[u])) : fma_rn(av[u], xv[u], acc);
+      }
       ep.store(r, acc);
     }
     __syncwarp();
@@ -180,7 +189,7 @@ __device__ __forceinline__ void spmv_bundle_h(const BundleHead& h, const int* __
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int e = e0 + u * 32 + lane;
-      if (e < cnt) stage[e] = EXACT ? mul_rn(mul_rn(alpha, av[u]), xv[u]) : xv[u];
+      if (e < cnt) stage[e] = EXACT ? mul_rn(UNIT ? av[u] : mul_rn(alpha, av[u]), xv[u]) : xv[u];
       if (!EXACT && GB_SPMV_STAGE_A && e < cnt) stage[kBundleNnz / 2 + e] = av[u];
     }
   }
@@ -202,16 +211,16 @@ __device__ __forceinline__ void spmv_bundle_h(const BundleHead& h, const int* __
   __syncwarp();
 }
 
-template <typename T, bool EXACT, typename XF, typename EP>
+template <typename T, bool EXACT, bool UNIT = true, typename XF, typename EP>
 __device__ __forceinline__ void spmv_bundle(int b, int n, const int* __restrict__ bundles,
                                             const int* __restrict__ ia, const int* __restrict__ ja,
                                             const T* __restrict__ a, T alpha, XF& xf, EP& ep, T* stage) {
-  spmv_bundle_h<T, EXACT>(bundle_head(b, n, bundles, ia), ia, ja, a, alpha, xf, ep, stage);
+  spmv_bundle_h<T, EXACT, UNIT>(bundle_head(b, n, bundles, ia), ia, ja, a, alpha, xf, ep, stage);
 }
 
 // Bundles b0, b0 + step, ... < nb, each bundle's head loaded while the one
 // before it is worked on.
-template <typename T, bool EXACT, typename XF, typename EP>
+template <typename T, bool EXACT, bool UNIT = true, typename XF, typename EP>
 __device__ __forceinline__ void spmv_bundles(int b0, int step, int nb, int n, const int* __restrict__ bundles,
                                              const int* __restrict__ ia, const int* __restrict__ ja,
                                              const T* __restrict__ a, T alpha, XF& xf, EP& ep, T* stage) {
@@ -220,7 +229,7 @@ __device__ __forceinline__ void spmv_bundles(int b0, int step, int nb, int n, co
   for (int b = b0; b < nb; b += step) {
     const int bn = b + step;
     const BundleHead hn = bn < nb ? bundle_head(bn, n, bundles, ia) : h;
-    spmv_bundle_h<T, EXACT>(h, ia, ja, a, alpha, xf, ep, stage);
+    spmv_bundle_h<T, EXACT, UNIT>(h, ia, ja, a, alpha, xf, ep, stage);
     h = hn;
   }
 }
