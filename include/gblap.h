@@ -252,6 +252,13 @@ int gb_debug_step_plan(int n, const int *ia_host, const int *ja_host, int lower,
                        int *info, int *tiles, unsigned short *ends, unsigned *meta, int *src,
                        unsigned short *needs, unsigned short *thr);
 
+/* Test hook (host only): the value-polling solve plan of the strict lower /
+ * upper part of a full CSR pattern.  info: {records, parts, levels}.  The
+ * arrays (NULL: sizes only): col, out, vsrc, dsrc [records * 32], lanes
+ * [records]; vsrc indexes the CSR's entries, dsrc its rows. */
+int gb_debug_flow_plan(int n, const int *ia_host, const int *ja_host, int lower, int *info, int *col, int *out,
+                       int *vsrc, int *dsrc, int *lanes);
+
 /* ------------------------------------------------------------ measurement */
 /* Per-kernel device times (ms per launch, CUDA events on the system stream)
  * of one PCG iteration's kernels, averaged over `iters` iterations run

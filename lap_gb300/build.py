@@ -21,7 +21,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libgblap.so")
 
-SOURCES = ["kernels.cu", "sptrsv.cu", "tri_plan.cu", "tri_step.cu", "pcg.cu", "precond.cu", "system.cu", "lap_abi.cu",
+SOURCES = ["kernels.cu", "sptrsv.cu", "tri_plan.cu", "tri_step.cu", "tri_flow.cu", "pcg.cu", "precond.cu", "system.cu", "lap_abi.cu",
            "lap_host.cu", "extras.cu", "batch.cu", "team.cu", "noalloc.cu", "mmio.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 

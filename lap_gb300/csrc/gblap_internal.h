@@ -103,8 +103,22 @@ struct StepPlan {
   unsigned *ticket = nullptr;
 };
 
+// Value-polling form (tri_flow.h): factors with many or far dependencies.
+struct FlowPlan {
+  bool on = false;
+  int elem = 0;  // bytes of a value: 4 or 8
+  int n = 0, nrec = 0, nslots = 0;
+  int *col = nullptr, *out = nullptr;    // [nrec * 32]
+  int *lanes = nullptr;                  // [nrec]
+  int *vsrc = nullptr, *dsrc = nullptr;  // [nrec * 32]
+  void *val = nullptr, *dinv = nullptr;  // [nrec * 32]
+  void *part = nullptr;                  // [nslots]
+  unsigned *ticket = nullptr;
+};
+
 struct TriPlan {
   StepPlan step;
+  FlowPlan flow;
   int n = 0;
   bool lower = true;
   int nlevels = 0;           // global dependency depth (diagnostics)

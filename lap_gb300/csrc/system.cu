@@ -18,6 +18,7 @@
 #include "pcg.h"
 #include "pcg_state.cuh"
 #include "sptrsv.h"
+#include "tri_flow.h"
 #include "tri_step.h"
 #include "system.h"
 
@@ -321,7 +322,7 @@ extern "C" int gb_system_create(int n, int nnz, const int* ia, const int* ja, co
     // The plans are independent host work (levels, packing, layout), built on
     // parallel threads, each with this thread's device current (4.19M-row
     // Chung-Lu: 8.8 s one after another).  An FP64 factor has two: the exact
-    // solves' records and, where the factor allows it, the lock-step form.
+    // solves' records and the PCG's form.
     {
       int dev = 0;
       CKC(cudaGetDevice(&dev));
@@ -642,8 +643,10 @@ static int solve_internal(gb_system s, const gb_pcg_opts* oin, gb_pcg_result* re
   const gb_pcg_opts* o = &oc;
   GB_TRY(system_ensure_hist(s, o->maxit));
   GB_CUDA_TRY(cudaMemsetAsync(s->err, 0, sizeof(int), s->s));
-  for (TriPlan* p : {o->precision == 0 ? &s->L : &s->L32, o->precision == 0 ? &s->U : &s->U32})
+  for (TriPlan* p : {o->precision == 0 ? &s->L : &s->L32, o->precision == 0 ? &s->U : &s->U32}) {
     GB_TRY(step_plan_reset(&p->step, s->s));
+    GB_TRY(flow_plan_reset(&p->flow, s->s));
+  }
   gb_pcg_result r;
   memset(&r, 0, sizeof r);
   PcgState* hs = s->st_host;

@@ -57,6 +57,7 @@
 #include "gb_common.cuh"
 #include "kernels.h"
 #include "spmv_bundle.cuh"
+#include "tri_flow.cuh"
 
 namespace gb {
 
@@ -1157,6 +1158,8 @@ int tri_launch_short(const TriPlan& p, const TriArgs<T>& A, OP op, cudaStream_t 
 
 template <typename T, typename OP, bool EXACT>
 int tri_launch(const TriPlan& p, const TriArgs<T>& A, OP op, cudaStream_t s) {
+  if constexpr (!EXACT)
+    if (p.flow.on) return flow_launch<T, OP>(p.flow, A.y, A.err, op, s);
   // split hub rows: every partial-sum slot at the sentinel before the solve
   if (p.nslots > 0) GB_TRY(fill_sentinel_dev(p.nslots, A.part, s));
   // The short-record kernel: FP64 for short-only plans; FP32 exactly for the

@@ -9,6 +9,7 @@
 #include "kernels.h"
 #include "sptrsv.h"
 #include "tri_kernel.cuh"
+#include "tri_flow.h"
 #include "tri_step.h"
 
 namespace gb {
@@ -191,7 +192,7 @@ void free_set(RecordSet* rs) {
 static bool record_form_forced() {
   for (const char* e : {"GBLAP_TRI_FORM", "GBLAP_TRI_SHORT", "GBLAP_TRI_FIXED", "GBLAP_TRI_CLUSTER",
                         "GBLAP_TRI_FP64_CLUSTER", "GBLAP_TRI_TILE_ROWS", "GBLAP_TRI_TILE_ROWS32",
-                        "GBLAP_TRI_BLOCKS_PER_SM"})
+                        "GBLAP_TRI_BLOCKS_PER_SM", "GBLAP_TRI_LEVEL_RUN", "GBLAP_TRI_PART_DEPS"})
     if (getenv(e)) return true;
   return false;
 }
@@ -212,17 +213,25 @@ static int row_levels(const TriDeps& d, std::vector<int>* out) {
   return nlev;
 }
 
+// What the PCG solves with: the lock-step form where it is allowed, else the
+// value-polling form.  Microseconds per solve (lower, FP64 / FP32), records
+// -> value polling: 131k-row Chung-Lu 594 / 549 -> 157 / 115, 1k-row 157 / 136
+// -> 54 / 33, 200k-row kNN 86 / 69 -> 74 / 50, 27-point 64^3 1510 / 1525 ->
+// 490 / 383, 12 x 12 x 100 1680 / 1912 -> 429 / 345, a band of 12 on 4000 rows
+// 5148 / 6096 -> 2675 / 2067: the records are left nowhere.
 int tri_step_plan_build(const TriDeps& d, TriPlan* plan, int elem) {
   if (record_form_forced()) return GB_OK;
   std::vector<int> lev;
   const int nlev = row_levels(d, &lev);
   GB_TRY(step_plan_build(d, lev, nlev, elem, &plan->step));
-  if (plan->step.on && elem == 4) {  // nothing else reads this plan
+  if (!plan->step.on) GB_TRY(flow_plan_build(d, elem, &plan->flow));
+  if ((plan->step.on || plan->flow.on) && elem == 4) {  // nothing else reads this plan
     plan->n = d.n;
     plan->lower = d.lower;
     plan->nlevels = nlev;
     plan->ntiles = plan->step.ntiles;
     plan->tile_rows = plan->step.tile_rows;
+    plan->levels_form = plan->flow.on;
     plan->ndeps = (long long)d.dep_col.size();
   }
   return GB_OK;
@@ -230,7 +239,7 @@ int tri_step_plan_build(const TriDeps& d, TriPlan* plan, int elem) {
 
 int tri_plan_build_fp32(const TriDeps& d, TriPlan* plan, int tile_rows, int level_run) {
   GB_TRY(tri_step_plan_build(d, plan, 4));
-  return plan->step.on ? GB_OK : tri_plan_build(d, plan, tile_rows, level_run);
+  return plan->step.on || plan->flow.on ? GB_OK : tri_plan_build(d, plan, tile_rows, level_run);
 }
 
 int tri_plan_build(const TriDeps& d, TriPlan* plan, int tile_rows, int level_run) {
@@ -455,6 +464,7 @@ int tri_plan_build(const TriDeps& d, TriPlan* plan, int tile_rows, int level_run
 
 void tri_plan_free(TriPlan* p) {
   step_plan_free(&p->step);
+  flow_plan_free(&p->flow);
   free_set(&p->r64);
   free_set(&p->r32);
   if (p->buf64s) cudaFree(p->buf64s);
@@ -546,13 +556,14 @@ int tri_default_tile_rows32(int n) {
 
 int tri_plan_fill(TriPlan* p, const double* ent_src, const double* diag_src, int mode,
                   cudaStream_t s) {
-  if (p->step.on && mode != kFillExact) {
-    GB_TRY(step_plan_fill(&p->step, ent_src, diag_src, s));
+  if ((p->step.on || p->flow.on) && mode != kFillExact) {
+    if (p->step.on) GB_TRY(step_plan_fill(&p->step, ent_src, diag_src, s));
+    else GB_TRY(flow_plan_fill(&p->flow, ent_src, diag_src, s));
     if (mode == kFillFma32) {
       p->have32 = true;
       return GB_OK;
     }
-    mode = kFillExact;  // the exact solves' records; the FMA form is the step plan's
+    mode = kFillExact;  // the exact solves' records; the FMA form is the other plan's
   }
   const int g = std::max(1, std::min(device_sm_count() * 8, ceil_div(std::max(p->nval, p->ndiag), 256)));
   fill_records_kernel<double><<<g, 256, 0, s>>>(p->nval, p->r64.vdst, p->vsrc, ent_src, p->ndiag,

@@ -501,15 +501,14 @@ int step_solve(const StepPlan& p, const TR* rhs, T* y, const int* done, int* err
   GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, (const StepArgs<T>)A, rhs));
   return GB_OK;
 }
-// The host layout for the strict one-sided part of a full CSR pattern.
-int step_layout_debug(int n, const int* ia, const int* ja, int lower, int elem, int tile_rows, int* info, int* tiles,
-                      unsigned short* ends, unsigned* meta, int* src, unsigned short* needs, unsigned short* thr) {
+TriDeps deps_of_part(int n, const int* ia, const int* ja, bool lower) {
   TriDeps d;
   d.n = n;
-  d.lower = lower != 0;
+  d.lower = lower;
   d.row_ptr.assign(n + 1, 0);
-  d.diag_src.assign(n, 0);
+  d.diag_src.resize(n);
   for (int i = 0; i < n; ++i) {
+    d.diag_src[i] = i;
     for (int k = ia[i]; k < ia[i + 1]; ++k)
       if ((lower && ja[k] < i) || (!lower && ja[k] > i)) {
         d.dep_col.push_back(ja[k]);
@@ -517,6 +516,13 @@ int step_layout_debug(int n, const int* ia, const int* ja, int lower, int elem, 
       }
     d.row_ptr[i + 1] = (int)d.dep_col.size();
   }
+  return d;
+}
+
+// The host layout for the strict one-sided part of a full CSR pattern.
+int step_layout_debug(int n, const int* ia, const int* ja, int lower, int elem, int tile_rows, int* info, int* tiles,
+                      unsigned short* ends, unsigned* meta, int* src, unsigned short* needs, unsigned short* thr) {
+  const TriDeps d = deps_of_part(n, ia, ja, lower != 0);
   std::vector<int> lev(n, 0);
   int nlev = 0;
   for (int q = 0; q < n; ++q) {

@@ -61,6 +61,10 @@ struct StepTile {
   int thr0;    // first of its chunks' thresholds
 };
 
+// The strict one-sided part of a full CSR pattern (the plans' test hooks);
+// diag_src is the row.
+TriDeps deps_of_part(int n, const int* ia, const int* ja, bool lower);
+
 // Builds the plan for values of `elem` bytes where the factor allows it
 // (every row within kStepDeps dependencies, all within one tile or the tile
 // before, shared memory for the previous tile's exports); plan->on says.
