@@ -44,7 +44,7 @@ struct SpmvPlan {
   int n = 0, nnz = 0;
   int nbundles = 0;
   int *bundles = nullptr;   // device [nbundles+1]
-  int long_rows = 0;        // diagnostics
+  int longest = 0;          // entries of the longest row
   int rows_per_bundle = kBundleRows;
 };
 

@@ -61,12 +61,12 @@ int spmv_plan_build(int n, int nnz, const int* ia, SpmvPlan* plan, int rpb) {
   std::vector<int> b;
   b.reserve(n / rpb + 2);
   b.push_back(0);
-  int r = 0, longs = 0;
+  int r = 0, longest = 0;
+  for (int i = 0; i < n; ++i) longest = std::max(longest, ia[i + 1] - ia[i]);
   while (r < n) {
     const int len0 = ia[r + 1] - ia[r];
     if (len0 > cap) {
       ++r;
-      ++longs;
       b.push_back(r);
       continue;
     }
@@ -83,12 +83,12 @@ int spmv_plan_build(int n, int nnz, const int* ia, SpmvPlan* plan, int rpb) {
   plan->n = n;
   plan->nnz = nnz;
   plan->nbundles = (int)b.size() - 1;
-  plan->long_rows = longs;
+  plan->longest = longest;
   plan->rows_per_bundle = rpb;
   // every bundle 32 consecutive rows (a stencil): the kernels' plan-free
   // layout computes the same bundles, one dependent load fewer per bundle.
   // Every reader of SpmvPlan::bundles takes nullptr as that layout.
-  bool uniform = rpb == kBundleRows && longs == 0;
+  bool uniform = rpb == kBundleRows && longest <= cap;
   for (size_t i = 0; uniform && i + 1 < b.size(); ++i)
     if (b[i] != (int)(i * kBundleRows)) uniform = false;
   if (uniform) {

@@ -130,8 +130,10 @@ __global__ void __launch_bounds__(kThreads)
 // Five resident blocks per SM, as spmv_pq_split_kernel: the FP64 form then
 // holds 48 registers with a 72-byte spill instead of 64 (128^3: 69.0 ->
 // 62.4 us); the FP32 form needs 48 either way.
-template <typename T, int WK>
-__global__ void __launch_bounds__(kThreads, 5)
+// LONG, for a matrix with a row of more than kSpmvSerial entries, needs more
+// registers and runs four.
+template <typename T, int WK, bool LONG>
+__global__ void __launch_bounds__(kThreads, LONG ? 4 : 5)
     spmv_pq_kernel(int n, int nb, const int* __restrict__ bundles, const int* __restrict__ ia,
                    const int* __restrict__ ja, const T* __restrict__ a, const T* __restrict__ w,
                    T* p, T* q, T* tfill, PcgState* st, double* part,
@@ -172,7 +174,7 @@ __global__ void __launch_bounds__(kThreads, 5)
   } ep{w, p, q, tfill, beta, first, 0.0, T(0), T(0), T(0)};
   const int wid = threadIdx.x >> 5;
   for (int bb = blockIdx.x * (kThreads / 32) + wid; bb < nb; bb += gridDim.x * (kThreads / 32))
-    spmv_bundle<T, false>(bb, n, bundles, ia, ja, a, T(1), xf, ep, stage[wid]);
+    spmv_bundle<T, false, true, LONG>(bb, n, bundles, ia, ja, a, T(1), xf, ep, stage[wid]);
   double acc[1] = {ep.pq};
   if (reduce_last<1>(acc, part, gridDim.x, blockIdx.x, &st->tk[TK_PQ], sm) && threadIdx.x == 0)
     st->pq = acc[0];
@@ -427,7 +429,8 @@ __global__ void __launch_bounds__(kThreads)
 // Five resident blocks per SM (at most 51 registers, no spills; 64 without
 // the bound): this latency-bound kernel needs the warps (128^3: 48.3 ->
 // 45.6 us; six or eight blocks spill and measured 48.1 / 53.1 us).
-__global__ void __launch_bounds__(kThreads, 5)
+template <bool LONG>
+__global__ void __launch_bounds__(kThreads, LONG ? 4 : 5)
     spmv_pq_split_kernel(int n, int nb, const int* __restrict__ bundles, const int* __restrict__ ia,
                          const int* __restrict__ ja, const float* __restrict__ a,
                          const float* __restrict__ w, double* p, double* q, float* tfill,
@@ -470,7 +473,7 @@ __global__ void __launch_bounds__(kThreads, 5)
   // each bundle's head loaded while the previous bundle is worked on (128^3:
   // 45.9 -> 44.7 us; the FP64 kernel, which then spills more, measured
   // slower with it: 62.1 -> 68 us)
-  spmv_bundles<float, false>(blockIdx.x * (kThreads / 32) + wid, gridDim.x * (kThreads / 32), nb, n, bundles, ia, ja,
+  spmv_bundles<float, false, true, LONG>(blockIdx.x * (kThreads / 32) + wid, gridDim.x * (kThreads / 32), nb, n, bundles, ia, ja,
                              a, 1.0f, xf, ep, stage[wid]);
   double acc[1] = {ep.pq};
   if (reduce_last<1>(acc, part, gridDim.x, blockIdx.x, &st->tk[TK_PQ], sm) && threadIdx.x == 0)
@@ -603,7 +606,7 @@ __global__ void __launch_bounds__(kThreads)
 // buffer, kThreads/32 x kBundleNnz x sizeof(T)).
 template <typename T>
 static int grid_for_bundles(int nb) {
-  return wave_grid(spmv_pq_kernel<T, WK_PREC>, kThreads, ceil_div(nb, kThreads / 32));
+  return wave_grid(spmv_pq_kernel<T, WK_PREC, false>, kThreads, ceil_div(nb, kThreads / 32));
 }
 static int grid_ew(int n) { return std::max(1, std::min(ceil_div(n, kThreads), reduction_grid())); }
 
@@ -792,7 +795,7 @@ static int launch_upper_split(gb_system sys, PcgState* st) {
 }
 
 static int grid_split(int nb) {
-  return wave_grid(spmv_pq_split_kernel, kThreads, ceil_div(nb, kThreads / 32));
+  return wave_grid(spmv_pq_split_kernel<false>, kThreads, ceil_div(nb, kThreads / 32));
 }
 
 // w = M^-1 r for the current FP64 r (the lower solve's output is pre-filled
@@ -818,7 +821,9 @@ int launch_body_split(gb_system sys, PcgState* st, cudaGraphConditionalHandle co
   auto& v = sys->v64;
   const int nb = sys->plan.nbundles;
   const float* w = sys->prec == GB_PREC_ICHOL ? sys->v32.s : sys->v32.w;
-  spmv_pq_split_kernel<<<grid_split(nb), kThreads, 0, sys->s>>>(
+  const bool rows_long = sys->plan.longest > kSpmvSerial;
+  auto pq = rows_long ? spmv_pq_split_kernel<true> : spmv_pq_split_kernel<false>;
+  pq<<<rows_long ? std::min(grid_split(nb), wave_grid(pq, kThreads, ceil_div(nb, kThreads / 32))) : grid_split(nb), kThreads, 0, sys->s>>>(
       sys->n, nb, sys->plan.bundles, sys->ia, sys->ja, sys->a32, w, v.p0, v.q,
       sys->L32.step.on ? nullptr : sys->v32.t, st,
       sys->part, cond, has_cond);
@@ -865,11 +870,14 @@ int launch_body(gb_system sys, PcgState* st, cudaGraphConditionalHandle cond, in
   const T* a = mat_vals<T>(sys);
   const T* dr = dr_vals<T>(sys);
   const T* wbuf = w_buffer<T>(sys);
+  const bool rows_long = sys->plan.longest > kSpmvSerial;
 #define GB_PQ(WKV)                                                                             \
-  spmv_pq_kernel<T, WKV><<<g, kThreads, 0, sys->s>>>(sys->n, nb, sys->plan.bundles, sys->ia,   \
-                                                     sys->ja, a, wbuf, v.p0, v.q,               \
-                                                     tri && !step ? v.t : nullptr, st, sys->part, cond,  \
-                                                     has_cond)
+  do {                                                                                         \
+    auto pq = rows_long ? spmv_pq_kernel<T, WKV, true> : spmv_pq_kernel<T, WKV, false>;        \
+    const int gq = rows_long ? std::min(g, wave_grid(pq, kThreads, ceil_div(nb, kThreads / 32))) : g; \
+    pq<<<gq, kThreads, 0, sys->s>>>(sys->n, nb, sys->plan.bundles, sys->ia, sys->ja, a, wbuf, v.p0, v.q, \
+                                    tri && !step ? v.t : nullptr, st, sys->part, cond, has_cond); \
+  } while (0)
   if (wk == WK_NONE) GB_PQ(WK_NONE);
   else if (wk == WK_JACOBI) GB_PQ(WK_JACOBI);
   else GB_PQ(WK_PREC);

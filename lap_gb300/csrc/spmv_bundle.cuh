@@ -51,6 +51,14 @@ __device__ __forceinline__ void ep_prefetch(EP&, int, long) {}
 // Values of a row held in registers from the start of its bundle (FMA
 // form): a stencil row's whole dependency list is in flight at once.
 constexpr int kSpmvHeld = 8;
+// LONG (FMA form), for matrices with rows of more than kSpmvSerial entries:
+// entries a lane sums by itself at most, and gathers of a lane in flight in a
+// row too long to stage.  131k-row Chung-Lu (a row of 11k entries), one
+// spmv_pq: 118 -> 67 us in FP64, 59 -> 34 us in split precision; 3k rows 40 ->
+// 21 us.  Bound by the longest row's chain of gathers.  A kernel of its own:
+// in the others its registers would spill (FP64 spmv_pq 72 -> 260 bytes).
+constexpr int kSpmvSerial = 32;
+constexpr int kSpmvBatch = 8;
 // 1: bundles whose rows all have at most kSpmvHeld entries take the
 // per-lane form (no staging).
 #ifndef GB_SPMV_SHORT_ROWS
@@ -95,10 +103,11 @@ __device__ __forceinline__ BundleHead bundle_head(int b, int n, const int* __res
   return h;
 }
 
-template <typename T, bool EXACT, bool UNIT, typename XF, typename EP>
+template <typename T, bool EXACT, bool UNIT, bool LONG, typename XF, typename EP>
 __device__ __forceinline__ void spmv_bundle_h(const BundleHead& h, const int* __restrict__ ia,
                                               const int* __restrict__ ja, const T* __restrict__ a, T alpha, XF& xf,
                                               EP& ep, T* stage) {
+  static_assert(!LONG || (!EXACT && !GB_SPMV_STAGE_A), "long rows are summed in another order");
   const int lane = threadIdx.x & 31;
   const int r0 = h.r0, r1 = h.r1;
   const int nr = r1 - r0;
@@ -116,9 +125,36 @@ __device__ __forceinline__ void spmv_bundle_h(const BundleHead& h, const int* __
     for (int rr = r0; rr < r1; ++rr) {
       const int k0 = __ldg(ia + rr), k1 = __ldg(ia + rr + 1);
       T s = T(0);
-      for (int j = k0 + lane; j < k1; j += 32) {
-        const T xv = xf(__ldg(ja + j));
-        s = EXACT ? add_rn(s, mul_rn(UNIT ? __ldg(a + j) : mul_rn(alpha, __ldg(a + j)), xv)) : fma_rn(__ldg(a + j), xv, s);
+      if constexpr (!LONG) {
+        for (int j = k0 + lane; j < k1; j += 32) {
+          const T xv = xf(__ldg(ja + j));
+          s = EXACT ? add_rn(s, mul_rn(UNIT ? __ldg(a + j) : mul_rn(alpha, __ldg(a + j)), xv)) : fma_rn(__ldg(a + j), xv, s);
+        }
+      } else {
+        // kSpmvBatch gathers of a lane in flight and the next columns behind
+        // them: a hub row has thousands of entries, each an L2 round trip
+        int c[kSpmvBatch];
+        auto columns = [&](int j) {
+#pragma unroll
+          for (int u = 0; u < kSpmvBatch; ++u) c[u] = j + 32 * u < k1 ? __ldg(ja + j + 32 * u) : -1;
+        };
+        columns(k0 + lane);
+        T s1 = T(0);
+        for (int j = k0 + lane; j < k1; j += 32 * kSpmvBatch) {
+          T av[kSpmvBatch], xv[kSpmvBatch];
+#pragma unroll
+          for (int u = 0; u < kSpmvBatch; ++u) {
+            av[u] = c[u] >= 0 ? __ldg(a + j + 32 * u) : T(0);
+            xv[u] = c[u] >= 0 ? xf(c[u]) : T(0);
+          }
+          columns(j + 32 * kSpmvBatch);
+#pragma unroll
+          for (int u = 0; u < kSpmvBatch; u += 2) {
+            s = fma_rn(av[u], xv[u], s);
+            s1 = fma_rn(av[u + 1], xv[u + 1], s1);
+          }
+        }
+        s = add_rn(s, s1);
       }
       s = warp_sum(s);
       if (lane == 0) {
@@ -194,7 +230,25 @@ __device__ __forceinline__ void spmv_bundle_h(const BundleHead& h, const int* __
     }
   }
   __syncwarp();
-  if (own) {
+  // LONG: a long row is summed by the whole warp -- alone, its lane
+  // would add its entries one FP64 latency after another while the pipe
+  // issues for the other lanes' idle slots too
+  bool mine = own;
+  if constexpr (LONG) {
+    unsigned lng = __ballot_sync(0xffffffffu, own && re - rs > kSpmvSerial);
+    if (lng & (1u << lane)) mine = false;
+    while (lng) {
+      const int src = __ffs(lng) - 1;
+      lng &= lng - 1u;
+      const int e1 = __shfl_sync(0xffffffffu, re, src) - j0;
+      T s = T(0);
+      for (int e = __shfl_sync(0xffffffffu, rs, src) - j0 + lane; e < e1; e += 32)
+        s = fma_rn(__ldg(a + j0 + e), stage[e], s);
+      s = warp_sum(s);
+      if (lane == src) ep.store(r, add_rn(acc, s));
+    }
+  }
+  if (mine) {
     const int e0 = rs - j0, e1 = re - j0;
     if (EXACT) {
       for (int e = e0; e < e1; ++e) acc = add_rn(acc, stage[e]);
@@ -211,16 +265,16 @@ __device__ __forceinline__ void spmv_bundle_h(const BundleHead& h, const int* __
   __syncwarp();
 }
 
-template <typename T, bool EXACT, bool UNIT = true, typename XF, typename EP>
+template <typename T, bool EXACT, bool UNIT = true, bool LONG = false, typename XF, typename EP>
 __device__ __forceinline__ void spmv_bundle(int b, int n, const int* __restrict__ bundles,
                                             const int* __restrict__ ia, const int* __restrict__ ja,
                                             const T* __restrict__ a, T alpha, XF& xf, EP& ep, T* stage) {
-  spmv_bundle_h<T, EXACT, UNIT>(bundle_head(b, n, bundles, ia), ia, ja, a, alpha, xf, ep, stage);
+  spmv_bundle_h<T, EXACT, UNIT, LONG>(bundle_head(b, n, bundles, ia), ia, ja, a, alpha, xf, ep, stage);
 }
 
 // Bundles b0, b0 + step, ... < nb, each bundle's head loaded while the one
 // before it is worked on.
-template <typename T, bool EXACT, bool UNIT = true, typename XF, typename EP>
+template <typename T, bool EXACT, bool UNIT = true, bool LONG = false, typename XF, typename EP>
 __device__ __forceinline__ void spmv_bundles(int b0, int step, int nb, int n, const int* __restrict__ bundles,
                                              const int* __restrict__ ia, const int* __restrict__ ja,
                                              const T* __restrict__ a, T alpha, XF& xf, EP& ep, T* stage) {
@@ -229,7 +283,7 @@ __device__ __forceinline__ void spmv_bundles(int b0, int step, int nb, int n, co
   for (int b = b0; b < nb; b += step) {
     const int bn = b + step;
     const BundleHead hn = bn < nb ? bundle_head(bn, n, bundles, ia) : h;
-    spmv_bundle_h<T, EXACT, UNIT>(h, ia, ja, a, alpha, xf, ep, stage);
+    spmv_bundle_h<T, EXACT, UNIT, LONG>(h, ia, ja, a, alpha, xf, ep, stage);
     h = hn;
   }
 }
