@@ -120,15 +120,29 @@ __device__ __forceinline__ void for_bundles(const BatchArgs& B, F&& body) {
 }
 
 // Fixed-order sum of NV interleaved partials part[stride*i + k], i in
-// [i0, i1), by the whole block; valid in thread 0.
+// [i0, i1), by the whole block; valid in thread 0.  A thread's loads go out
+// eight at a time: one after another they were most of the reduction (80^3,
+// 32 right-hand sides, 6,080 partials each: alpha 20 -> 9, check 23 ->
+// 14 us).
 template <int NV>
 __device__ __forceinline__ void block_segment_sum(const double* part, int stride, int i0, int i1,
                                                   double (&v)[NV], double* sm) {
 #pragma unroll
   for (int k = 0; k < NV; ++k) v[k] = 0.0;
-  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x)
+  constexpr int U = 8;
+  for (int i = i0 + threadIdx.x; i < i1; i += U * blockDim.x) {
+    double t[U][NV];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) v[k] += part[(size_t)stride * i + k];
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int k = 0; k < NV; ++k)
+        t[u][k] = i + u * (int)blockDim.x < i1 ? part[(size_t)stride * (i + u * (int)blockDim.x) + k] : 0.0;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i + u * (int)blockDim.x < i1)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) v[k] += t[u][k];
+  }
   block_sum<NV>(v, sm);
 }
 
@@ -693,8 +707,11 @@ __global__ void __launch_bounds__(kBatchThreads)
 // x += alpha p, r -= alpha q, w = M^-1 r; partials r'r, r'w per (system,
 // warp) at part_c[2 * (s * Wu + warp)], Wu = this grid's warps (its own,
 // larger than the row kernels').  Each lane takes kIlUpd row steps per pass,
-// all their loads issued before any store.
-constexpr int kIlUpd = 2;
+// all their loads issued before any store (80^3, 32 right-hand sides, an
+// iteration: 436 / 429 / 417 us with 1 / 2 / 4); the grid leaves a warp at
+// least kIlUpdSteps of them.
+constexpr int kIlUpd = 4;
+constexpr int kIlUpdSteps = 2;
 
 __global__ void __launch_bounds__(kBatchThreads) bil_update_kernel(BatchArgs B) {
   const IlLane L(B);
@@ -756,14 +773,17 @@ __global__ void __launch_bounds__(kBatchThreads) bil_alpha_kernel(BatchArgs B) {
   PcgState& O = B.so[s];
   const bool repl = il_replaces(B, s);
   if (!repl && S.done) return;  // uniform in the block
-  double v[3];
-  block_segment_sum<3>(B.part_b, 3, s * B.nb, (s + 1) * B.nb, v, sm);
-  if (threadIdx.x != 0) return;
   if (repl) {
+    double v[3];
+    block_segment_sum<3>(B.part_b, 3, s * B.nb, (s + 1) * B.nb, v, sm);
+    if (threadIdx.x != 0) return;
     outer_decide(B, S, O, v[0], v[1], B.delta, B.max_outer);
     B.rep[s] = 1;
     return;
   }
+  double v[1];  // p'q alone: FP64 adds are what the reduction is made of
+  block_segment_sum<1>(B.part_b, 3, s * B.nb, (s + 1) * B.nb, v, sm);
+  if (threadIdx.x != 0) return;
   S.pq = v[0];
   double alpha;
   if (!pcg_alpha(&S, &alpha)) {
@@ -1452,7 +1472,7 @@ int multi_batch(gb_system sys, gb_batch* slot, int nrhs, bool interleaved, gb_ba
       const long long steps = ((long long)sys->n + 32 / nrhs - 1) / (32 / nrhs);
       bt->il_ugrid = (int)std::max(
           1LL, std::min((long long)device_sm_count() * occupancy_blocks((const void*)bil_update_kernel, kBatchThreads),
-                        (steps + kBatchWarps * kIlUpd - 1) / (kBatchWarps * kIlUpd)));
+                        (steps + kBatchWarps * kIlUpdSteps - 1) / (kBatchWarps * kIlUpdSteps)));
       const int wu = bt->il_ugrid * kBatchWarps;
       bt->nc = wu * nrhs;
       std::vector<int> sc(nrhs + 1);
