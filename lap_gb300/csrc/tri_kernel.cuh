@@ -969,6 +969,9 @@ __global__ void __launch_bounds__((TriCons<T, SHORT>::threads), 1) tri_tile_kern
     }
     if constexpr (CL > 1) cluster_sync_all();  // the group's pushes are complete
   }
+  // the last ticket was read from rank 0's shared memory: no CTA of the cluster
+  // leaves before all have read it
+  if constexpr (CL > 1) cluster_sync_all();
   // Drain: every issued copy must have landed before the CTA's shared
   // memory goes away.  A slot is refilled only after its previous record was
   // consumed, so only the last copy into each slot can still be in flight
