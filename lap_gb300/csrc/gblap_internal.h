@@ -107,7 +107,7 @@ struct StepPlan {
 struct FlowPlan {
   bool on = false;
   int elem = 0;  // bytes of a value: 4 or 8
-  int n = 0, nrec = 0, nslots = 0;
+  int n = 0, nrec = 0, nslots = 0, nlev = 0;
   int *col = nullptr, *out = nullptr;    // [nrec * 32]
   int *lanes = nullptr;                  // [nrec]
   int *vsrc = nullptr, *dsrc = nullptr;  // [nrec * 32]

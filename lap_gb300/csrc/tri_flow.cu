@@ -127,6 +127,7 @@ int flow_plan_build(const TriDeps& d, int elem, FlowPlan* plan) {
   plan->n = d.n;
   plan->nrec = L.nrec;
   plan->nslots = L.nslots;
+  plan->nlev = L.nlev;
   GB_TRY(upload(&plan->col, L.col));
   GB_TRY(upload(&plan->out, L.out));
   GB_TRY(upload(&plan->lanes, L.lanes));

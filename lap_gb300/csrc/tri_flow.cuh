@@ -152,7 +152,12 @@ int flow_launch(const FlowPlan& p, T* y, int* err, OP op, cudaStream_t s) {
   F.ticket = p.ticket;
   F.err = err;
   constexpr int warps = kFlowThreads / 32;
-  const int grid = std::max(1, std::min((p.nrec + warps - 1) / warps, device_sm_count()));
+  // Two blocks an SM where a level holds more than half of one block's records
+  // an SM (FP64 lower solve of 1M-row Chung-Lu 444 -> 340 us, 800k-row kNN 199
+  // -> 150, 200k-row 73 -> 62), one where levels are narrow and more warps only
+  // poll (131k-row Chung-Lu 157 either way, 20k-row kNN 37 against 39 us).
+  const int per_sm = 2LL * p.nrec > (long long)p.nlev * warps * device_sm_count() ? 2 : 1;
+  const int grid = std::max(1, std::min((p.nrec + warps - 1) / warps, per_sm * device_sm_count()));
   tri_flow_kernel<T, OP><<<grid, kFlowThreads, 0, s>>>(F, op);
   GB_CUDA_TRY(cudaGetLastError());
   return GB_OK;

@@ -216,7 +216,7 @@ static int row_levels(const TriDeps& d, std::vector<int>* out) {
 // What the PCG solves with: the lock-step form where it is allowed, else the
 // value-polling form.  Microseconds per solve (lower, FP64 / FP32), records
 // -> value polling: 131k-row Chung-Lu 594 / 549 -> 157 / 115, 1k-row 157 / 136
-// -> 54 / 33, 200k-row kNN 86 / 69 -> 74 / 50, 27-point 64^3 1510 / 1525 ->
+// -> 54 / 33, 200k-row kNN 86 / 69 -> 62 / 45, 27-point 64^3 1510 / 1525 ->
 // 490 / 383, 12 x 12 x 100 1680 / 1912 -> 429 / 345, a band of 12 on 4000 rows
 // 5148 / 6096 -> 2675 / 2067: the records are left nowhere.
 int tri_step_plan_build(const TriDeps& d, TriPlan* plan, int elem) {

@@ -63,6 +63,26 @@ def test_matches_records_and_oracle(name, prec, monkeypatch):
     rec.close()
 
 
+@pytest.mark.parametrize("precision", [0, 2])
+def test_wide_levels(precision, monkeypatch):
+    """A level of thousands of records (two blocks an SM), against the records
+    and reproducible; the bounds above."""
+    A = gen.knn_graph(100000, 8, seed=4)
+    b = torch.from_numpy(np.random.default_rng(8).uniform(-1.0, 1.0, A.n)).cuda()
+    s = gb.System.from_csr(A, "ichol")
+    monkeypatch.setenv("GBLAP_TRI_FORM", "levels")
+    rec = gb.System.from_csr(A, "ichol")
+    x, r = s.solve(b, tol=1e-12, maxit=20000, precision=precision)
+    y, q = rec.solve(b, tol=1e-12, maxit=20000, precision=precision)
+    assert r["flag"] == q["flag"] == 0 and r["status"] == q["status"] == 0
+    assert abs(r["iters"] - q["iters"]) <= max(1, int(np.ceil(0.02 * q["iters"])))
+    assert float(torch.linalg.norm(x - y) / torch.linalg.norm(y)) < 1e-8
+    again, _ = s.solve(b, tol=1e-12, maxit=20000, precision=precision)
+    assert torch.equal(again, x)
+    s.close()
+    rec.close()
+
+
 def test_a_wait_that_runs_out():
     """A chain of 150 rows a tile apart, each on the five before it, among
     rows of their own: the far ones wait for more than two clock checks.  With
