@@ -505,380 +505,14 @@ def run_workload(args, local):
     print(json.dumps(line), flush=True)
 
 
-def run_ours(args, world, rank, local):
-    import torch
-
-    import lap_gb300 as gb
-
-    torch.cuda.set_device(local)
-    A, b = make_workload(args.size)
-    n, nnz = A.n, A.nnz
-    sysm = gb.System.from_csr(A, "ichol")
-    info = sysm.info()
-    db = torch.from_numpy(b).cuda()
-    kw = dict(tol=args.tol, maxit=20000)
-
-    # warm-up: graphs captured, clocks up
-    for _ in range(args.warmup):
-        sysm.solve(db, precision=MIXED, **kw)
-        sysm.solve(db, precision=0, **kw)
-    sysm.solve(db, precision=1, **kw)
-
-    def timed(precision, steps):
-        ms, res = [], None
-        barrier(world)
-        torch.cuda.synchronize()
-        for _ in range(steps):
-            x, res = sysm.solve(db, precision=precision, **kw)
-            ms.append(res["device_ms"])
-        torch.cuda.synchronize()
-        barrier(world)
-        return ms, res, x
-
-    with ClockSampler(local) as clk:
-        t0 = time.time()
-        ms_mixed, r_mixed, x_mixed = timed(MIXED, args.steps)
-        wall = time.time() - t0
-    ms_fp64, r_fp64, x_fp64 = timed(0, max(2, args.steps // 2))
-    ms_f32k, r_f32k, x_f32k = timed(1, 2)
-    err_vs_fp64 = float(torch.linalg.norm(x_mixed - x_fp64) / torch.linalg.norm(x_fp64))
-
-    # end to end from pinned host buffers
-    bh = torch.from_numpy(b).pin_memory()
-    xh = torch.zeros(n, dtype=torch.float64).pin_memory()
-    e2e = []
-    for _ in range(args.steps):
-        xh.zero_()
-        r = gb.PcgResult()
-        o = gb.opts(precision=MIXED, **kw)
-        gb.check(gb.lib().gb_pcg_solve_host(sysm.h, bh.data_ptr(), xh.data_ptr(), gb.C.byref(o),
-                                            gb.C.byref(r)), "gb_pcg_solve_host")
-        e2e.append(r.device_ms)
-
-    # per-kernel device time of one iteration (CUDA events on the solver stream)
-    peak, peak_kind = measured_peak()
-    pname = {0: "fp64", 1: "fp32-krylov", 2: "split"}
-    prof = {p: sysm.profile(db, precision=p, iters=20) for p in (0, 1, 2)}
-    traffic = ncu_traffic()
-    kernels = []
-    for p, lst in prof.items():
-        for k in lst:
-            gbs = k["bytes"] / (k["ms"] * 1e-3) / 1e9 if k["ms"] > 0 else 0.0
-            kernels.append({"kernel": k["name"], "precision": pname[p],
-                            "ms": round(k["ms"], 5), "bytes": k["bytes"], "gbs": round(gbs, 1),
-                            "frac": round(gbs / peak, 4)})
-    src = f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else "fallback 6.8 TB/s"
-
-    def roof(k):
-        return {"bound": "hbm", "kernel": k["kernel"], "precision": k["precision"],
-                "achieved": k["gbs"], "peak": peak, "unit": "GB/s", "frac": k["frac"],
-                "traffic": traffic.get(f"{k['kernel']}:{k['precision']}"), "peak_source": src}
-
-    mixed_k = [k for k in kernels if k["precision"] == pname[MIXED]]
-    dom = max(mixed_k, key=lambda k: k["ms"])  # a triangular solve: dependency-latency bound
-    roofline = roof(dom)
-    # the bandwidth-bound kernels of the same iteration (SpMV + fused vector updates)
-    bw = {k["kernel"]: roof(k) for k in kernels
-          if k["precision"] in ("fp64", pname[MIXED]) and k["kernel"] in ("spmv_pq", "spmv_pq_split", "update")}
-
-    v = allmax(world, statistics.mean(ms_mixed))
-    v64 = allmax(world, statistics.mean(ms_fp64))
-    v32k = allmax(world, statistics.mean(ms_f32k))
-    ve2e = allmax(world, statistics.mean(e2e))
-    if rank != 0:
-        return
-    it_in, outer = r_mixed["iters"], r_mixed["outer"]
-    # our kernels per split solve: the fills of the two solves' mailboxes; the
-    # first FP64 residual; the prologue (residual, the two triangular solves,
-    # r'w); 5 per iteration (SpMV, update, the two solves, r'w); per replacement
-    # its FP64 residual and, unless it ends the solve, the resume (state reset,
-    # solves, r'w); the final true residual
-    launches_mixed = 2 + 1 + 4 + 5 * it_in + outer + 4 * max(outer - 1, 0) + 1
-    line = {"metric": METRIC, "value": round(v, 1), "unit": UNIT, "impl": "reference", "n_gpus": args.gpus,
-            "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(v, 1), "higher_is_better": False,
-            "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
-            "config": {"workload": WORKLOAD + " (reference: FP64 IC0-PCG, CPU)", "iterations": iters[-1],
-                       "flag": r["flag"], "steps_ms": [round(t, 1) for t in times]},
-            "cpu_baseline": {"value": round(v, 1), "unit": UNIT, "cores": max(spmv_t, dot_t), "kind": "port",
-                             "sample": f"one full solve per step ({iters[-1]} iterations, cg() only as LAP's "
-                                       f"Time line); restatement of LAP's OpenMP backend: SpMV on {spmv_t} "
-                                       f"threads (openmp_blas.c:37), dot on {dot_t}, serial triangular solves",
-                             "host": host_info()},
-            "e2e": {"value": round(v, 1), "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
-            "wall_s": round(time.time() - t0, 1)}
-    print(json.dumps(line), flush=True)
-
-
-def run_kernels_only(args, local):
-    """Per-kernel device times of PCG iterations run eagerly (no graph), for
-    each precision mode -- the launches a profiler can attribute one by one."""
-    import torch
-
-    import lap_gb300 as gb
-
-    torch.cuda.set_device(local)
-    A, b = make_workload(args.size)
-    sysm = gb.System.from_csr(A, "ichol")
-    db = torch.from_numpy(b).cuda()
-    precs = [int(t) for t in args.profile_precisions.split(",")]
-    out = {p: [(k["name"], round(k["ms"], 5)) for k in sysm.profile(db, precision=p, iters=args.profile_iters)]
-           for p in precs}
-    print(json.dumps({"kernels_only": out, "n": A.n, "nnz": A.nnz}), flush=True)
-
-
-def _timed_solves(fn, steps):
-    import torch
-
-    out = []
-    for _ in range(steps):
-        torch.cuda.synchronize()
-        out.append(fn())
-    return out
-
-
-def _edge_positions(A, ei, ej):
-    """CSR positions of each edge's two entries and of every diagonal, and the
-    index of each edge among A's strict-lower entries (row-major)."""
-    rows = np.repeat(np.arange(A.n), np.diff(A.ia))
-    key = rows.astype(np.int64) * A.n + A.ja
-    lo, hi = np.minimum(ei, ej), np.maximum(ei, ej)
-    strict_lower = np.nonzero(A.ja < rows)[0]
-    p_lh = np.searchsorted(key, lo * A.n + hi)
-    p_hl = np.searchsorted(key, hi * A.n + lo)
-    diag = np.searchsorted(key, np.arange(A.n, dtype=np.int64) * (A.n + 1))
-    return lo, hi, p_lh, p_hl, diag, np.searchsorted(strict_lower, p_hl)
-
-
-def run_workload(args, local):
-    """The other configurations at full size (256^2 Jacobi, Chung-Lu, the
-    kNN batch, multi-RHS, the adjoint, the Matrix Market read; parity cases
-    beside the headline bench line): one JSON line each with times and
-    accuracy."""
-    import torch
-
-    import lap_gb300 as gb
-    from lap_gb300 import gen
-
-    torch.cuda.set_device(local)
-    wl = args.workload
-    line = {"workload": wl, "data": "synthetic (seeded generator)"}
-    t0 = time.time()
-    if wl == "jacobi256":
-        import oracle
-
-        A, b = gen.grid2d_unit(256, seed=1001)
-        line["config"] = "256^2 unit 5-point + 1e-2 I, line_jacobi, tol 1e-8, maxit 10000 (FP64)"
-        sysm = gb.System.from_csr(A, "line_jacobi")
-        db = torch.from_numpy(b).cuda()
-        for _ in range(3):
-            sysm.solve(db, tol=1e-8, maxit=10000)
-        res = _timed_solves(lambda: sysm.solve(db, tol=1e-8, maxit=10000), 5)
-        x, r = res[-1]
-        ref = oracle.solve(A.n, A.ia, A.ja, A.a, b, "line_jacobi", 1e-8, 10000)
-        line.update(ms=statistics.mean(rr["device_ms"] for _, rr in res), iters=r["iters"],
-                    ref_iters=ref["iters"], rel_true_res=r["rel_true_res"],
-                    x_rel_err_vs_reference=float(np.linalg.norm(x.cpu().numpy() - ref["x"]) /
-                                                 np.linalg.norm(ref["x"])),
-                    cpu_reference_ms=ref["solve_s"] * 1e3, cpu_cores=1)
-    elif wl == "mmread128":
-        import ctypes as C
-        import tempfile
-
-        A, _ = gen.grid3d_lognormal(128, seed=1002)
-        line["config"] = ("128^3 lognormal Laplacian written as 'coordinate real symmetric' (lower triangle, "
-                          "%.17g values), read into CSR: host read_mm_file + coo_to_csr vs gb_mm_read_csr")
-        with tempfile.TemporaryDirectory() as td:
-            path = os.path.join(td, "g128.mtx")
-            tw = time.time()
-            gen.write_mm(path, A)
-            line["file_bytes"] = os.path.getsize(path)
-            line["write_s"] = round(time.time() - tw, 1)
-            L = gb.lib()
-            gb.read_mm_device(path)  # warm-up (module load, first allocations)
-            runs = []
-            for _ in range(3):
-                torch.cuda.synchronize()
-                t1 = time.perf_counter()
-                ia, ja, a, info = gb.read_mm_device(path)
-                runs.append((time.perf_counter() - t1, info))
-            wall, info = min(runs, key=lambda t: t[0])
-            line["device"] = {"wall_ms": round(wall * 1e3, 1), "read_ms": round(info["read_ms"], 1),
-                              "h2d_ms": round(info["h2d_ms"], 2), "device_ms": round(info["device_ms"], 2),
-                              "device_gbs_of_file": round(line["file_bytes"] / info["device_ms"] / 1e6, 1),
-                              "host_parsed": info["host_parsed"], "nnz": info["nnz"]}
-            M = gb.MMatrix()
-            t1 = time.perf_counter()
-            L.read_mm_file(path.encode(), C.byref(M))
-            L.coo_to_csr(C.byref(M))
-            line["host_reader_ms"] = round((time.perf_counter() - t1) * 1e3, 1)
-            hia = np.ctypeslib.as_array(M.csr_ia, (M.n + 1,)).copy()
-            hja = np.ctypeslib.as_array(M.csr_ja, (M.nnz_unpacked,)).copy()
-            ha = np.ctypeslib.as_array(M.csr_vals, (M.nnz_unpacked,)).copy()
-            libc = C.CDLL(None)
-            for q in (M.csr_ia, M.csr_ja, M.csr_vals):
-                libc.free(C.cast(q, C.c_void_p))
-            line["identical_to_host_reader"] = bool(
-                np.array_equal(ia.cpu().numpy(), hia) and np.array_equal(ja.cpu().numpy(), hja)
-                and np.array_equal(a.cpu().numpy().view(np.int64), ha.view(np.int64)))
-            line["identical_to_generator"] = bool(
-                np.array_equal(hia, A.ia) and np.array_equal(hja, A.ja) and np.array_equal(ha, A.a))
-            line["speedup_vs_host_reader"] = round(line["host_reader_ms"] / (wall * 1e3), 1)
-    elif wl == "chunglu4m":
-        A, b = gen.chung_lu(1 << 22, seed=1003)
-        line["config"] = f"Chung-Lu n={A.n} nnz={A.nnz}, A=1.001 D - W, ichol, tol 1e-10"
-        line["generate_s"] = round(time.time() - t0, 1)
-        t1 = time.time()
-        sysm = gb.System.from_csr(A, "ichol")
-        line["setup_s"] = round(time.time() - t1, 1)
-        line["levels"] = sysm.info()
-        db = torch.from_numpy(b).cuda()
-        kw = dict(tol=1e-10, maxit=20000)
-        x64, r64 = sysm.solve(db, precision=0, **kw)
-        for p in (0, 1, 2):
-            sysm.solve(db, precision=p, **kw)
-            x, r = sysm.solve(db, precision=p, **kw)
-            line[f"precision{p}"] = {"ms": round(r["device_ms"], 2), "iters": r["iters"], "outer": r["outer"],
-                                     "flag": r["flag"], "rel_true_res": r["rel_true_res"],
-                                     "rel_err_vs_fp64": float(torch.linalg.norm(x - x64) / torch.linalg.norm(x64))}
-        # the mode chosen by timing (gb_pcg_autotune_precision), then a solve in it
-        tune = sysm.autotune_precision(db, **kw)
-        sysm.solve(db, precision=-1, **kw)
-        res = _timed_solves(lambda: sysm.solve(db, precision=-1, **kw), 3)
-        x, r = res[-1]
-        line["autotune_precision"] = {"best": tune["best"], "ms_per_mode": [round(v, 2) for v in tune["ms"]],
-                                      "solve_ms": round(statistics.mean(rr["device_ms"] for _, rr in res), 2),
-                                      "iters": r["iters"],
-                                      "rel_err_vs_fp64": float(torch.linalg.norm(x - x64) / torch.linalg.norm(x64))}
-    elif wl == "batch512":
-        mats, rhs = gen.knn_batch(512, seed=1004)
-        line["config"] = (f"512 kNN(k=8) Laplacians, n log-uniform 1k-200k (sum n = {sum(A.n for A in mats)}, "
-                          f"sum nnz = {sum(A.nnz for A in mats)}), line_jacobi, tol 1e-8, one graph launch")
-        line["generate_s"] = round(time.time() - t0, 1)
-        bt = gb.Batch(mats, "line_jacobi")
-        db = torch.from_numpy(np.concatenate(rhs)).cuda()
-        x64, i64, f64, r64 = bt.solve(db, tol=1e-8, maxit=20000, precision=0)
-        for p in (0, 2):
-            bt.solve(db, tol=1e-8, maxit=20000, precision=p)
-            res = _timed_solves(lambda: bt.solve(db, tol=1e-8, maxit=20000, precision=p), 3)
-            x, its, fl, r = res[-1]
-            line[f"precision{p}"] = {"ms": round(statistics.mean(rr["device_ms"] for *_, rr in res), 2),
-                                     "max_iters": int(its.max()), "all_converged": bool((fl == 0).all()),
-                                     "rel_true_res_max": r["rel_true_res"],
-                                     "rel_err_vs_fp64": float(torch.linalg.norm(x - x64) / torch.linalg.norm(x64))}
-        # the autotuner's plan for this batch, then the same solves on it
-        tune = bt.autotune(db, iters=16)
-        line["autotune"] = dict(tune)
-        for p in (0, 2):
-            bt.solve(db, tol=1e-8, maxit=20000, precision=p)
-            res = _timed_solves(lambda: bt.solve(db, tol=1e-8, maxit=20000, precision=p), 3)
-            x, its, fl, r = res[-1]
-            line["autotune"][f"precision{p}_ms"] = round(statistics.mean(rr["device_ms"] for *_, rr in res), 2)
-            line["autotune"][f"precision{p}_all_converged"] = bool((fl == 0).all())
-            line["autotune"][f"precision{p}_rel_err_vs_fp64"] = float(torch.linalg.norm(x - x64) /
-                                                                      torch.linalg.norm(x64))
-        t2 = time.time()  # the same systems one by one with the single-system solver
-        ms = 0.0
-        for A, b in zip(mats, rhs):
-            sg = gb.System.from_csr(A, "line_jacobi")
-            _, rs = sg.solve(torch.from_numpy(b).cuda(), tol=1e-8, maxit=20000)
-            ms += rs["device_ms"]
-            sg.close()
-        line["one_by_one_device_ms"] = round(ms, 2)
-        line["one_by_one_wall_s"] = round(time.time() - t2, 1)
-    elif wl in ("multirhs32", "multirhs64"):
-        nr = int(wl[len("multirhs"):])
-        A, _ = gen.grid3d_lognormal(128, seed=1002)
-        Bm = torch.from_numpy(gen.multi_rhs(A.n, nr, seed=1005)).cuda()
-        line["config"] = (f"128^3 lognormal Laplacian, {nr} RHS, line_jacobi, tol 1e-8, "
-                          + ("one graph launch" if nr <= 32 else "chunks of 32 RHS, one graph launch each"))
-        sysm = gb.System.from_csr(A, "line_jacobi")
-        X64, i64, _ = gb.solve_multi(sysm, Bm, tol=1e-8, maxit=20000, precision=0)
-        forms = [("", None)] + ([("blocks_", "blocks")] if nr > 32 else [])
-        for tag, form in forms:
-            if form:  # every column in one launch on concatenated vectors
-                os.environ["GBLAP_MULTI_FORM"] = form
-            for p in (0, 2):
-                gb.solve_multi(sysm, Bm, tol=1e-8, maxit=20000, precision=p)
-                X, its, r = gb.solve_multi(sysm, Bm, tol=1e-8, maxit=20000, precision=p)
-                line[f"{tag}precision{p}"] = {
-                    "ms": round(r["device_ms"], 2), "max_iters": int(its.max()), "flag": r["flag"],
-                    "rel_true_res_max": r["rel_true_res"],
-                    "rel_err_vs_fp64": float(torch.linalg.norm(X - X64) / torch.linalg.norm(X64))}
-            os.environ.pop("GBLAP_MULTI_FORM", None)
-        tune = gb.autotune_multi(sysm, Bm, iters=16)  # columns per interleaved chunk, by timing
-        line["autotune"] = dict(tune)
-        for p in (0, 2):
-            gb.solve_multi(sysm, Bm, tol=1e-8, maxit=20000, precision=p)
-            X, its, r = gb.solve_multi(sysm, Bm, tol=1e-8, maxit=20000, precision=p)
-            line["autotune"][f"precision{p}_ms"] = round(r["device_ms"], 2)
-            line["autotune"][f"precision{p}_rel_err_vs_fp64"] = float(torch.linalg.norm(X - X64) /
-                                                                      torch.linalg.norm(X64))
-        ms = 0.0
-        for k in range(Bm.shape[0]):
-            _, rs = sysm.solve(Bm[k], tol=1e-8, maxit=20000)
-            ms += rs["device_ms"]
-        line["one_by_one_device_ms"] = round(ms, 2)
-    elif wl == "adjoint1024":
-        nside = 1024
-        ei, ej, w = gen.grid2d_aniso_edges(nside, seed=1006)
-        A = gen.laplacian_from_edges(nside * nside, ei, ej, w, shift=1e-2)
-        rng = np.random.default_rng(1006)
-        xs = torch.from_numpy(rng.standard_normal(A.n)).cuda()
-        b = torch.from_numpy(rng.uniform(-1, 1, A.n)).cuda()
-        line["config"] = ("1024^2 anisotropic lognormal grid + 1e-2 I, ichol, loss 0.5||x-x*||^2; forward and "
-                          "adjoint in split precision (tol 1e-10); central differences h=1e-6 (FP64, tol 1e-13) "
-                          "and the reference CPU PCG's own adjoint (FP64 IC(0), tol 1e-10) on the same random edges")
-        sysm = gb.System.from_csr(A, "ichol")
-        kw = dict(tol=1e-10, maxit=20000, precision=2)
-        sysm.solve(b, **kw)
-        x, rf = sysm.solve(b, **kw)
-        lam, G, eg, ra = sysm.adjoint(x, (x - xs).contiguous(), **kw)
-        line["forward_ms"], line["adjoint_ms"] = round(rf["device_ms"], 2), round(ra["device_ms"], 2)
-        line["iters"] = [rf["iters"], ra["iters"]]
-        lo, hi, p_lh, p_hl, diag, t_of_edge = _edge_positions(A, ei, ej)
-        a0 = torch.from_numpy(A.a).cuda()
-        edges = np.random.default_rng(1007).choice(len(w), args.fd_edges, replace=False)
-        fds, ads = [], []
-        for e in edges:
-            vals = []
-            for sgn in (1.0, -1.0):
-                a = a0.clone()
-                d = sgn * 1e-6
-                a[int(p_lh[e])] -= d
-                a[int(p_hl[e])] -= d
-                a[int(diag[lo[e]])] += d
-                a[int(diag[hi[e]])] += d
-                sysm.set_values(a)
-                xe, _ = sysm.solve(b, tol=1e-13, maxit=50000, precision=0)
-                vals.append(0.5 * float(torch.sum((xe - xs) ** 2)))
-            fds.append((vals[0] - vals[1]) / 2e-6)
-            ads.append(float(eg[int(t_of_edge[e])]))
-        sysm.set_values(a0)
-        fds, ads = np.array(fds), np.array(ads)
-        line["fd_edges"] = int(args.fd_edges)
-        line["fd_abs_err_max_over_max_grad"] = float(np.abs(fds - ads).max() / np.abs(ads).max())
-        line["fd_rel_err_median"] = float(np.median(np.abs(fds - ads) / np.abs(ads)))
-        # the reference's CPU PCG (the oracle, FP64 IC(0)) for the forward and
-        # the adjoint solve; its gradient on the same edges and its dL/db
-        import oracle
-
-        t2 = time.time()
-        bn, xsn = b.cpu().numpy(), xs.cpu().numpy()
-        ref_f = oracle.solve(A.n, A.ia, A.ja, A.a, bn, "ichol", 1e-10, 20000)
-        ref_a = oracle.solve(A.n, A.ia, A.ja, A.a, ref_f["x"] - xsn, "ichol", 1e-10, 20000)
-        xr, lr = ref_f["x"], ref_a["x"]
-        g_ref = np.array([-(lr[lo[e]] - lr[hi[e]]) * (xr[lo[e]] - xr[hi[e]]) for e in edges])
-        lam_np = lam.cpu().numpy()
-        line["reference_adjoint"] = {
-            "iters": [ref_f["iters"], ref_a["iters"]], "cpu_s": round(time.time() - t2, 1),
-            "grad_abs_err_max_over_max_grad": float(np.abs(ads - g_ref).max() / np.abs(g_ref).max()),
-            "grad_rel_err_median": float(np.median(np.abs(ads - g_ref) / np.abs(g_ref))),
-            "dL_db_rel_err": float(np.linalg.norm(lam_np - lr) / np.linalg.norm(lr)),
-            "fd_vs_reference_grad_max_over_max_grad": float(np.abs(fds - g_ref).max() / np.abs(g_ref).max())}
-    else:
-        raise SystemExit(f"unknown workload {wl}")
-    line["wall_s"] = round(time.time() - t0, 1)
-    print(json.dumps(line), flush=True)
+def split_launches(iters, replacements):
+    """Our kernels of one split solve whose two triangular solves run in several
+    clusters (the headline system's do): the fills of their mailboxes; the
+    first FP64 residual; the prologue (residual, the two solves, r'w); five an
+    iteration (SpMV, update, the two solves, r'w); per replacement its FP64
+    residual and, unless it ends the solve, the resume (state reset, the two
+    solves, r'w); the final true residual."""
+    return 2 + 1 + 4 + 5 * iters + replacements + 4 * max(replacements - 1, 0) + 1
 
 
 def run_ours(args, world, rank, local):
@@ -964,17 +598,7 @@ def run_ours(args, world, rank, local):
     if rank != 0:
         return
     it_in, outer = r_mixed["iters"], r_mixed["outer"]
-    # our kernels per split-precision solve: first outer residual 1, prologue 4
-    # (residual, sentinel fill, lower, upper), 4 per iteration (one graph body:
-    # spmv_pq_split, update, lower, upper), an outer residual after each of the
-    # `outer` pauses, 4 per resume (resume, fill, lower, upper; all pauses but
-    # the last), final true residual 1
-    # our kernels per split solve: the first FP64 residual; the prologue
-    # (residual, sentinel fill, the two triangular solves, r'w); 5 per
-    # iteration (SpMV, update, the two solves, r'w); per replacement its
-    # FP64 residual and, unless it ends the solve, the resume (state reset,
-    # sentinel fill, solves, r'w); the final true residual
-    launches_mixed = 1 + 5 + 5 * it_in + outer + 5 * max(outer - 1, 0) + 1
+    launches_mixed = split_launches(it_in, outer)
     line = {"metric": METRIC, "value": round(v, 4), "unit": UNIT, "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(v, 4),
             "higher_is_better": False, "scaling": "weak", "vs_baseline": None,
