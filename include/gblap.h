@@ -240,6 +240,13 @@ int gb_pcg_autotune_precision(gb_system sys, const double *b, const gb_pcg_opts 
  * returns, so the solve ends with status GB_TIMEOUT instead of hanging. */
 int gb_debug_set_spin_budget(gb_system sys, unsigned long long ns);
 
+/* Test hook: the one-launch recurrences of sys (or of batch, sys NULL) ask for
+ * at least this much shared memory per block (0: what they need; at most
+ * 204,800 bytes).  Where the
+ * device then cannot hold all their blocks at once it refuses the launch, and
+ * the solve runs the captured loop instead. */
+int gb_debug_set_team_smem(gb_system sys, gb_batch batch, int bytes);
+
 /* Test hook (host only): the lock-step solve plan of the strict lower / upper
  * part of a full CSR pattern, for values of elem_bytes (4 or 8).  tile_rows 0:
  * the planner's choice.  info: {tiles, rows of a tile, solver warps, staged

@@ -108,6 +108,7 @@ def _proto(L: C.CDLL) -> None:
         "gb_pcg_autotune_multi": (i, [vp, i, vp, i, C.POINTER(i), C.POINTER(d), C.POINTER(d)]),
         "gb_pcg_autotune_precision": (i, [vp, vp, vp, C.POINTER(i), vp]),
         "gb_debug_set_spin_budget": (i, [vp, C.c_ulonglong]),
+        "gb_debug_set_team_smem": (i, [vp, vp, i]),
         "gb_debug_step_plan": (i, [i, vp, vp, i, i, i, vp, vp, vp, vp, vp, vp, vp]),
         "gb_debug_flow_plan": (i, [i, vp, vp, i, vp, vp, vp, vp, vp, vp]),
         "gb_dot_noalloc": (i, [i, vp, vp, C.POINTER(C.c_double), vp]),

@@ -1184,9 +1184,9 @@ int batch_loop(gb_batch bt, int split, int maxit, int use_graph) {
   if (bt->team.on && !bt->no_team) {
     TeamData<double, double> d{bt->ia, bt->ja, bt->a, bt->jacobi ? bt->d_r : nullptr, bt->x, bt->r, bt->w, bt->p, bt->q,
                                bt->row_off, bt->N, bt->st, nullptr, 0, bt->err};
-    if (!split) return team_loop(bt->team, d, bt->s);
     TeamData<double, float> f{d.ia, d.ja, bt->a32, d.d_r, d.x, d.r, d.w, d.p, d.q, d.row_off, d.n, d.st, nullptr, 0, d.err};
-    return team_loop(bt->team, f, bt->s);
+    const int rc = split ? team_loop(bt->team, f, bt->s) : team_loop(bt->team, d, bt->s);
+    if (rc != GB_NOT_SUPPORTED) return rc;  // the loop where the device refuses the launch
   }
   GB_CUDA_TRY(cudaMemsetAsync(bt->tk, 0, sizeof(unsigned) * 4, bt->s));
   GB_CUDA_TRY(cudaMemsetAsync(bt->nactive, 0, sizeof(int) * 4, bt->s));
@@ -1406,6 +1406,12 @@ extern "C" int gb_batch_create(int count, const long long* row_off_host, const l
   if ((rc = team_plan_build(count, bt->h_roff, bt->h_ia.data(), &bt->team)) != GB_OK) return fail(rc);
   if (hbad) return fail(GB_BAD_INPUT);  // a row without a (nonzero) diagonal
   *out = bt;
+  return GB_OK;
+}
+
+extern "C" int gb_debug_set_team_smem(gb_system sys, gb_batch bt, int bytes) {
+  if ((!sys && !bt) || bytes < 0 || (size_t)bytes > kTeamMaxSmem) return GB_BAD_INPUT;
+  (sys ? sys->team : bt->team).debug_smem = (size_t)bytes;
   return GB_OK;
 }
 

@@ -39,7 +39,6 @@ namespace gb {
 
 namespace {
 
-constexpr size_t kTeamMaxSmem = 200 * 1024;
 constexpr int kTeamWarps = kTeamThreads / 32;  // worker warps; one more does the scalars
 
 __device__ __forceinline__ void team_bar(int id) {
@@ -448,8 +447,13 @@ int team_loop(const TeamPlan& p, const TeamData<T, TA>& d, cudaStream_t s) {
   A.mail0 = p.mail0;
   A.cached = p.smem ? p.max_nnz : 0;
   void* args[] = {&A};
-  GB_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)team_kernel<T, TA>(p.rows), dim3(p.ctas), dim3(kTeamThreads + 32),
-                                          args, p.smem, s));
+  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)team_kernel<T, TA>(p.rows), dim3(p.ctas),
+                                                    dim3(kTeamThreads + 32), args, std::max(p.smem, p.debug_smem), s);
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported) {
+    cudaGetLastError();
+    return GB_NOT_SUPPORTED;
+  }
+  GB_CUDA_TRY(e);
   return GB_OK;
 }
 template int team_loop<double, double>(const TeamPlan&, const TeamData<double, double>&, cudaStream_t);

@@ -17,6 +17,7 @@ struct TeamPlan {
   int ctas = 0, rows = 0;   // blocks; rows of a thread (1 to 4)
   size_t smem = 0;          // bytes of matrix entries kept in shared memory (0: none)
   int max_nnz = 0;          // most entries of a block
+  size_t debug_smem = 0;    // test hook: bytes to ask for at least, past what the device gives every block
   int *cta_sys = nullptr, *cta0 = nullptr;  // device [ctas], [systems + 1]
   double *mail = nullptr;        // device: per system [blocks][4][blocks][2]
   long long *mail0 = nullptr;    // device [systems]
@@ -24,6 +25,7 @@ struct TeamPlan {
 };
 
 constexpr int kTeamThreads = 256;
+constexpr size_t kTeamMaxSmem = 200 * 1024;
 constexpr int kTeamMaxRow = 64;  // entries of a row (a thread sums its rows alone)
 
 // Plans `count` systems of rows [row_off[s], row_off[s+1]) with global row
@@ -50,6 +52,9 @@ struct TeamData {
 
 // Runs every system's recurrence from its state until it is done (or its
 // state says it is), as the loops of update / spmv_pq kernels do.
+// GB_NOT_SUPPORTED, with nothing of the state touched, where the device refuses
+// the launch (fewer SMs for this context than when the plan was made): the
+// caller then runs the loop.
 template <typename T, typename TA>
 int team_loop(const TeamPlan& plan, const TeamData<T, TA>& d, cudaStream_t s);
 
