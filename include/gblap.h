@@ -206,10 +206,12 @@ int gb_autotune_spmv(gb_system sys, int *best_host);
 /* Picks a block-diagonal batch's row-bundle and tile sizes by timing them:
  * rows per SpMV bundle in {32, 16, 8} x rows per update / reduction chunk in
  * {2048, 1024, 4096}, each running `iters` iterations (<= 0: 16) of the
- * batch's own captured solve loop (FP64, no stopping) on right-hand side b;
- * the fastest is applied to the batch and cached per matrix class (system
- * count, rows, entries, longest row), so later batches of that class are set
- * without timing.  Results of the tuned batch equal the default's up to the
+ * batch's own solve loop (FP64, no stopping) on right-hand side b; the
+ * fastest is applied to the batch and cached per matrix class (system count,
+ * rows, entries, longest row, kind of loop), so later batches of that class
+ * are set without timing.  A batch that fits the device's blocks at once runs
+ * its loop as one launch, which neither size reaches: the defaults 32 and 2048
+ * are timed, once, and kept.  Results of the tuned batch equal the default's up to the
  * rounding of the regrouped reductions.  Outputs may be NULL; the times are
  * 0 when the choice came from the cache.  GB_NOT_SUPPORTED for multi-RHS
  * batches (see gb_pcg_autotune_multi).  No counterpart in LAP. */

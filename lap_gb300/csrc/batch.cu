@@ -947,7 +947,6 @@ struct gb_batch_s {
   int chunk_rows = kChunkRows; // rows per update / reduction chunk
   size_t part_b_cap = 0, part_c_cap = 0;
   TeamPlan team;       // block-diagonal: every system's loop in one launch, where they fit
-  bool no_team = false;  // the autotuner times the bundle loop
   int* err = nullptr;  // [4] error word and spin budget of the team loop's waits
 };
 
@@ -1181,7 +1180,7 @@ int batch_body(gb_batch bt, int split, int maxit, cudaGraphConditionalHandle con
 
 // The iteration loop as one graph: a while node around batch_body.
 int batch_loop(gb_batch bt, int split, int maxit, int use_graph) {
-  if (bt->team.on && !bt->no_team) {
+  if (bt->team.on) {
     TeamData<double, double> d{bt->ia, bt->ja, bt->a, bt->jacobi ? bt->d_r : nullptr, bt->x, bt->r, bt->w, bt->p, bt->q,
                                bt->row_off, bt->N, bt->st, nullptr, 0, bt->err};
     TeamData<double, float> f{d.ia, d.ja, bt->a32, d.d_r, d.x, d.r, d.w, d.p, d.q, d.row_off, d.n, d.st, nullptr, 0, d.err};
@@ -1555,14 +1554,16 @@ extern "C" int gb_pcg_solve_multi(gb_system sys, int nrhs, const double* B, doub
 // ------------------------------------------------------------ autotuner
 // The batch's tile and row-bundle choices, picked by timing them: each
 // candidate runs `iters` iterations of the solve loop the batch really uses
-// (the captured CUDA-graph while loop, FP64, tol 0 so no system stops), and
-// the fastest is kept.  Choices are cached per matrix class, so a second
-// batch of the same shape is tuned without timing.
+// (FP64, tol 0 so no system stops), and the fastest is kept.  A batch whose
+// loop is one launch (team.cu) has neither tiles nor bundles in it: the
+// defaults are timed and kept.  Choices are cached per matrix class, so a
+// second batch of the same shape is tuned without timing.
 namespace {
 struct BatchClass {
   int count, N, nnz, maxrow;
+  bool team;  // system sizes decide it too
   bool operator<(const BatchClass& o) const {
-    return std::tie(count, N, nnz, maxrow) < std::tie(o.count, o.N, o.nnz, o.maxrow);
+    return std::tie(count, N, nnz, maxrow, team) < std::tie(o.count, o.N, o.nnz, o.maxrow, o.team);
   }
 };
 std::mutex g_btune_mu;
@@ -1598,15 +1599,10 @@ int batch_time(gb_batch bt, const double* b, double* x, int iters, double* ms) {
   o.tol = 0.0;
   o.maxit = iters;
   gb_pcg_result r;
-  bt->no_team = true;
-  int rc = GB_OK;
-  for (int k = 0; k < 2 && rc == GB_OK; ++k) {
-    rc = cudaMemsetAsync(x, 0, sizeof(double) * (size_t)bt->N, bt->s) == cudaSuccess
-             ? batch_solve(bt, b, x, &o, nullptr, nullptr, &r)
-             : GB_CUDA_ERROR;
+  for (int k = 0; k < 2; ++k) {
+    GB_CUDA_TRY(cudaMemsetAsync(x, 0, sizeof(double) * (size_t)bt->N, bt->s));
+    GB_TRY(batch_solve(bt, b, x, &o, nullptr, nullptr, &r));
   }
-  bt->no_team = false;
-  GB_TRY(rc);
   *ms = r.device_ms;
   return GB_OK;
 }
@@ -1619,7 +1615,7 @@ extern "C" int gb_batch_autotune(gb_batch bt, const double* b, int iters, int* r
   if (iters <= 0) iters = 16;
   int maxrow = 0;
   for (int i = 0; i < bt->N; ++i) maxrow = std::max(maxrow, bt->h_ia[i + 1] - bt->h_ia[i]);
-  const BatchClass key{bt->count, bt->N, bt->h_ia[bt->N], maxrow};
+  const BatchClass key{bt->count, bt->N, bt->h_ia[bt->N], maxrow, bt->team.on};
   std::pair<int, int> best{kBundleRows, kChunkRows};
   double t_def = 0.0, t_best = 0.0;
   bool cached = false;
@@ -1638,6 +1634,7 @@ extern "C" int gb_batch_autotune(gb_batch bt, const double* b, int iters, int* r
     t_best = 1e300;
     for (int rpb : {kBundleRows, 16, 8}) {
       for (int cr : {kChunkRows, 1024, 4096}) {
+        if (bt->team.on && (rpb != kBundleRows || cr != kChunkRows)) continue;
         double ms = 0.0;
         rc = batch_replan(bt, rpb, cr);
         if (rc == GB_OK) rc = batch_time(bt, b, x, iters, &ms);
