@@ -261,6 +261,10 @@ int gb_debug_step_plan(int n, const int *ia_host, const int *ja_host, int lower,
                        int *info, int *tiles, unsigned short *ends, unsigned *meta, int *src,
                        unsigned short *needs, unsigned short *thr);
 
+/* Test hook (host only): the form in which a PCG solves the strict lower /
+ * upper part of a full CSR pattern: 0 records, 1 lock-step, 2 value polling. */
+int gb_debug_tri_form(int n, const int *ia_host, const int *ja_host, int lower, int elem_bytes, int *form);
+
 /* Test hook (host only): the value-polling solve plan of the strict lower /
  * upper part of a full CSR pattern.  info: {records, parts, levels}.  The
  * arrays (NULL: sizes only): col, out, vsrc, dsrc [records * 32], lanes

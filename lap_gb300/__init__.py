@@ -110,6 +110,7 @@ def _proto(L: C.CDLL) -> None:
         "gb_debug_set_spin_budget": (i, [vp, C.c_ulonglong]),
         "gb_debug_set_team_smem": (i, [vp, vp, i]),
         "gb_debug_step_plan": (i, [i, vp, vp, i, i, i, vp, vp, vp, vp, vp, vp, vp]),
+        "gb_debug_tri_form": (i, [i, vp, vp, i, i, vp]),
         "gb_debug_flow_plan": (i, [i, vp, vp, i, vp, vp, vp, vp, vp, vp]),
         "gb_dot_noalloc": (i, [i, vp, vp, C.POINTER(C.c_double), vp]),
         "gb_mm_read_csr": (i, [C.c_char_p, C.POINTER(MmCsr)]),

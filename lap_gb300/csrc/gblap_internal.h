@@ -77,6 +77,7 @@ struct RecordSet {
 // Lock-step form of a factor (tri_step.h): built for factors whose rows have
 // few, near dependencies; the PCG's solves then run it instead of the records.
 struct StepPlan {
+  bool fits = false;  // the factor allows the form
   bool on = false;
   int elem = 0;       // bytes of a value: 4 or 8
   int k = 0;          // the most dependencies a row has (2, 3 or 4)

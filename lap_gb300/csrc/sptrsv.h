@@ -37,9 +37,9 @@ constexpr int kTriMaxTileRows32 = 32768;
 // level_run: records per run in the levels form (0: one per consumer warp
 // of an FP64 CTA; FP32 plans pass tri_consumer_warps(4))
 int tri_plan_build(const TriDeps& d, TriPlan* plan, int tile_rows = 0, int level_run = 0);
-// The PCG's form in values of `elem` bytes (4 or 8): plan->step where the
-// factor allows it (tri_step.h), else plan->flow (tri_flow.h); neither where a
-// record form is asked for.
+// The PCG's form in values of `elem` bytes (4 or 8), by estimated time:
+// plan->step (tri_step.h), plan->flow (tri_flow.h), or neither, which leaves
+// the records; neither too where a record form is asked for.
 int tri_step_plan_build(const TriDeps& d, TriPlan* plan, int elem);
 // The FP32 solves' plan: that form alone, or the records.
 int tri_plan_build_fp32(const TriDeps& d, TriPlan* plan, int tile_rows, int level_run);

@@ -213,18 +213,76 @@ static int row_levels(const TriDeps& d, std::vector<int>* out) {
   return nlev;
 }
 
-// What the PCG solves with: the lock-step form where it is allowed, else the
-// value-polling form.  Microseconds per solve (lower, FP64 / FP32), records
-// -> value polling: 131k-row Chung-Lu 594 / 549 -> 157 / 115, 1k-row 157 / 136
-// -> 54 / 33, 200k-row kNN 86 / 69 -> 62 / 45, 27-point 64^3 1510 / 1525 ->
-// 490 / 383, 12 x 12 x 100 1680 / 1912 -> 429 / 345, a band of 12 on 4000 rows
-// 5148 / 6096 -> 2675 / 2067: the records are left nowhere.
+// Most dependencies cross tiles: the records' levels form.
+static bool most_deps_cross(const TriDeps& d, int tile_rows) {
+  long long cross = 0;
+  for (int i = 0; i < d.n; ++i)
+    for (int k = d.row_ptr[i]; k < d.row_ptr[i + 1]; ++k) cross += d.dep_col[k] / tile_rows != i / tile_rows;
+  const long long total = (long long)d.dep_col.size();
+  return total > 0 && 2 * cross > total;
+}
+
+// Estimated microseconds of a value-polling solve, launch apart: a level's
+// round trip and its records' turn.  Measured levels (FP64 / FP32): 0.5 / 0.4
+// us on a path to 1.05 / 0.85 on 7-point grids, and about 70 ps a row where
+// levels are wide (160^3: 706 / 602 us).
+static double flow_estimate(int n, int nlev, int elem) { return (elem == 8 ? 0.9 : 0.75) * nlev + 7e-5 * n; }
+
+// Whether a factor that the lock-step form has no room for is faster on the
+// records: most dependencies inside the tile or a tile's length away, rows of
+// the short-record kernels, many levels and none too wide -- a level then
+// costs a shared-memory hand-off instead of an L2 round trip.  Records / value
+// polling, us (lower): 40000 x 6 FP64 13271 / 26952, FP32 7249 / 24212; 300 x
+// 300 x 10 327 / 641, 244 / 553; 600 x 600 x 10 989 / 1467, 561 / 1291; 250 x
+// 250 x 40 (4,647 rows a level) 719 / 728, 546 / 622; past 5,000 rows a level
+// 300 x 300 x 40 882 / 818, 733 / 703; 300 x 300 x 60 1269 / 945, 1022 / 817;
+// 192^3 FP64 1294 / 1035.  Planes that reach little past one tile stay faster
+// at twice that: 145^3 FP64 525 / 595, 148 x 148 x 300 881 / 988, but 160^3
+// (1.56 tiles) 712 / 706.  A single row of 20 among 240,000 in strips of
+// 40,000: 27784 / 46943, 28683 / 41426; six dependencies a row, 20 x 5000:
+// 10278 / 7925, 12435 / 6407; most of them crossing tiles, 9-point 40000 x 6:
+// 72668 / 28131.
+static bool records_faster(const TriDeps& d, int nlev) {
+  const int n = d.n, tile = tri_default_tile_rows(n);
+  int band = 0;
+  long long rows_long = 0;
+  for (int i = 0; i < n; ++i) {
+    const int b = d.row_ptr[i], e = d.row_ptr[i + 1];
+    if (e - b > kTriHeld) {
+      ++rows_long;
+      continue;
+    }
+    for (int k = b; k < e; ++k) band = std::max(band, std::abs(i - d.dep_col[k]));
+  }
+  const long long width = n / std::max(nlev, 1);
+  return nlev >= 32 && 1000 * rows_long <= n && width <= (2LL * band <= 3LL * tile ? 12000 : 5000) &&
+         !most_deps_cross(d, tile);
+}
+
+enum { kFormRecords = 0, kFormStep = 1, kFormFlow = 2 };
+
+// The form where lock step is not taken; step_fits: it was found slower, which
+// it is for few and wide levels only.
+static int form_without_step(const TriDeps& d, int nlev, bool step_fits) {
+  return step_fits || !records_faster(d, nlev) ? kFormFlow : kFormRecords;
+}
+
+// What the PCG solves with: the lock-step form where the factor allows it and
+// a solve is not estimated longer than by polling values; else value polling
+// or the records.  Step / polling / records, us (split lower): shuffled 100^2
+// 39 / 17 / 40, 200^2 118 / 20 / 44, red-black 100^2 33 / 8 / 16, a shuffled
+// path of 20,000 66 / 13 / 23, but 20^3 16 / 50 / 37, 100 x 100 27 / 128 / 57,
+// a hundred separate 30 x 30 grids 27 / 51 / 37.  Graphs of many dependencies a
+// row (records -> polling, FP64 / FP32): 131k-row Chung-Lu 594 / 549 -> 157 /
+// 115, 200k-row kNN 86 / 69 -> 62 / 45, 27-point 64^3 1510 / 1525 -> 490 / 383,
+// a band of 12 on 4000 rows 5148 / 6096 -> 2675 / 2067.
 int tri_step_plan_build(const TriDeps& d, TriPlan* plan, int elem) {
   if (record_form_forced()) return GB_OK;
   std::vector<int> lev;
   const int nlev = row_levels(d, &lev);
-  GB_TRY(step_plan_build(d, lev, nlev, elem, &plan->step));
-  if (!plan->step.on) GB_TRY(flow_plan_build(d, elem, &plan->flow));
+  GB_TRY(step_plan_build(d, lev, nlev, elem, flow_estimate(d.n, nlev, elem), &plan->step));
+  if (!plan->step.on && form_without_step(d, nlev, plan->step.fits) == kFormFlow)
+    GB_TRY(flow_plan_build(d, elem, &plan->flow));
   if ((plan->step.on || plan->flow.on) && elem == 4) {  // nothing else reads this plan
     plan->n = d.n;
     plan->lower = d.lower;
@@ -277,11 +335,7 @@ int tri_plan_build(const TriDeps& d, TriPlan* plan, int tile_rows, int level_run
   int nslots = 0;  // partial-sum slots of split hub rows
   bool levels_form = false;
   {
-    long long cross = 0;
-    for (int i = 0; i < n; ++i)
-      for (int k = d.row_ptr[i]; k < d.row_ptr[i + 1]; ++k) cross += d.dep_col[k] / tile_rows != i / tile_rows;
-    const long long total = (long long)d.dep_col.size();
-    levels_form = total > 0 && 2 * cross > total;
+    levels_form = most_deps_cross(d, tile_rows);
     if (const char* e = getenv("GBLAP_TRI_FORM")) {
       if (!strcmp(e, "levels")) levels_form = true;
       if (!strcmp(e, "tiles")) levels_form = false;
@@ -674,3 +728,15 @@ int tri_solve_plain(const TriPlan* p, const double* x, double* y, int* err, cuda
 }
 
 }  // namespace gb
+
+extern "C" int gb_debug_tri_form(int n, const int* ia_host, const int* ja_host, int lower, int elem_bytes, int* form) {
+  if (n <= 0 || !ia_host || !ja_host || !form || (elem_bytes != 4 && elem_bytes != 8)) return GB_BAD_INPUT;
+  const gb::TriDeps d = gb::deps_of_part(n, ia_host, ja_host, lower != 0);
+  std::vector<int> lev;
+  const int nlev = gb::row_levels(d, &lev);
+  const double step = gb::step_plan_estimate(d, lev, nlev, elem_bytes);
+  const bool fits = step >= 0.0;
+  *form = fits && step <= gb::flow_estimate(n, nlev, elem_bytes) ? gb::kFormStep
+                                                                 : gb::form_without_step(d, nlev, fits);
+  return GB_OK;
+}

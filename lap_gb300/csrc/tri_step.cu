@@ -106,11 +106,15 @@ constexpr double kHopCycles = 250.0;      // more for a step whose inputs come f
 constexpr double kCrossCycles = 2000.0;   // and from another cluster, through L2
 constexpr int kResidentTiles = 140;       // about what clusters of 8 to 16 place on 152 SMs
 
+// Tiles of a cluster, as far as can be said before the device is asked.
+int cluster_guess(int ntiles) { return ntiles <= 16 ? ntiles : ntiles <= 112 ? 16 : 10; }
+
 int warps_for(int width) { return width <= 32 ? 1 : width <= 64 ? 2 : width <= 128 ? 4 : kStepMaxWarps; }
 
 // The host image of a plan.
 struct StepLayout {
   int k = 0, ntiles = 0, tile_rows = 0, nw = 0, np = 0, window = 0, nexp_max = 0, max_steps = 0, max_pages = 0, max_chunks = 0;
+  int width = 1;  // widest level of a tile
   bool nat = false;
   long long npages = 0;
   size_t smem = 0;
@@ -162,7 +166,7 @@ std::vector<int> step_heights(const TriDeps& d, const std::vector<int>& lev, int
       span = std::max(span, hi - lo + 1);
       for (int i = r0; i < r1; ++i) count[lev[i]] = 0;
     }
-    const int cl = nt <= 16 ? nt : nt <= 112 ? 16 : 10;
+    const int cl = cluster_guess(nt);
     double cost = step_cycles(elem, width) * std::max(span, nlev) + kHopCycles * (nt - 1) +
                   kCrossCycles * ((nt + cl - 1) / cl - 1);
     // clusters that are not resident start when an earlier one has ended
@@ -175,6 +179,20 @@ std::vector<int> step_heights(const TriDeps& d, const std::vector<int>& lev, int
   std::vector<int> h;
   for (const Cand& c : cands) h.push_back(c.rows);
   return h;
+}
+
+// Estimated microseconds of a solve laid out so, launch apart: the chain of
+// steps, hops and crossings as above, but of the steps that there are (a wide
+// level is several), and a tile's own rows on their way into its SM, which a
+// tile of few steps waits for (1.3 ns a row).  Against measured, split lower
+// solves: shuffled 100^2 33 / 31, 200^2 111 / 110, red-black 100^2 30 / 25,
+// 20^3 14 / 8, 160^3 446 / 420 us; it errs upwards on grids.
+double step_estimate(const StepLayout& L, int n, int nlev, int elem) {
+  const int cl = cluster_guess(L.ntiles);
+  double cycles = step_cycles(elem, std::min(L.width, 32 * L.nw)) * std::max(nlev, L.max_steps) +
+                  kHopCycles * (L.ntiles - 1) + kCrossCycles * ((L.ntiles + cl - 1) / cl - 1);
+  if (L.ntiles > kResidentTiles) cycles *= 2.0;  // 148 x 148 x 300 took 1.0 times, 160^3 1.9, 1000 x 700 on 175 tiles 2.2
+  return cycles / 2000.0 + 0.0013 * std::min(L.tile_rows, n);
 }
 
 // Lays the factor out in tiles of R rows; false where that does not fit.
@@ -230,6 +248,7 @@ bool step_layout(const TriDeps& d, const std::vector<int>& lev, int nlev, int el
     L->max_chunks = std::max(L->max_chunks, step_chunks(t1 - t0));
     L->npages += L->tiles[q].npages;
   }
+  L->width = width;
   L->nw = warps_for(width);
   const int per = 32 * L->nw;
   std::vector<int> step_end(R);
@@ -319,12 +338,22 @@ bool step_layout(const TriDeps& d, const std::vector<int>& lev, int nlev, int el
 
 }  // namespace
 
-int step_plan_build(const TriDeps& d, const std::vector<int>& lev, int nlev, int elem, StepPlan* plan) {
+double step_plan_estimate(const TriDeps& d, const std::vector<int>& lev, int nlev, int elem) {
+  int kmax = 0;
+  StepLayout L;
+  for (int R : step_heights(d, lev, nlev, elem, &kmax))
+    if (step_layout(d, lev, nlev, elem, kmax, R, &L)) return step_estimate(L, d.n, nlev, elem);
+  return -1.0;
+}
+
+int step_plan_build(const TriDeps& d, const std::vector<int>& lev, int nlev, int elem, double limit_us, StepPlan* plan) {
   *plan = StepPlan();
   int kmax = 0;
   StepLayout L;
   for (int R : step_heights(d, lev, nlev, elem, &kmax)) {
     if (!step_layout(d, lev, nlev, elem, kmax, R, &L)) continue;
+    plan->fits = true;
+    if (step_estimate(L, d.n, nlev, elem) > limit_us) return GB_OK;
     plan->elem = elem;
     plan->k = L.k;
     plan->ntiles = L.ntiles;

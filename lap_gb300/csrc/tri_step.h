@@ -67,9 +67,12 @@ TriDeps deps_of_part(int n, const int* ia, const int* ja, bool lower);
 
 // Builds the plan for values of `elem` bytes where the factor allows it
 // (every row within kStepDeps dependencies, all within one tile or the tile
-// before, shared memory for the previous tile's exports); plan->on says.
+// before, shared memory for the previous tile's exports) and a solve is
+// estimated at limit_us or less; plan->fits and plan->on say.
 // lev: the rows' global levels, nlev of them.
-int step_plan_build(const TriDeps& d, const std::vector<int>& lev, int nlev, int elem, StepPlan* plan);
+int step_plan_build(const TriDeps& d, const std::vector<int>& lev, int nlev, int elem, double limit_us, StepPlan* plan);
+// That estimate; negative where the factor does not allow the form.
+double step_plan_estimate(const TriDeps& d, const std::vector<int>& lev, int nlev, int elem);
 void step_plan_free(StepPlan* plan);
 // Writes the coefficients and reciprocal diagonals from the value arrays.
 int step_plan_fill(const StepPlan* plan, const double* ent_src, const double* diag_src, cudaStream_t s);
