@@ -276,7 +276,8 @@ int gb_debug_flow_plan(int n, const int *ia_host, const int *ja_host, int lower,
 /* Per-kernel device times (ms per launch, CUDA events on the system stream)
  * of one PCG iteration's kernels, averaged over `iters` iterations run
  * eagerly.  names_host receives a ';'-separated list of kernel names,
- * ms_host[i] and bytes_host[i] the average time and algorithmic bytes. */
+ * ms_host[i] and bytes_host[i] the average time and algorithmic bytes.
+ * GB_TIMEOUT where a wait of one of them gave up. */
 int gb_profile_iteration(gb_system sys, const double *b, double *x, int precision, int iters,
                          char *names_host, int names_len, double *ms_host,
                          double *bytes_host, int max_kernels, int *count);

@@ -194,7 +194,9 @@ extern "C" int gb_profile_iteration(gb_system s, const double* b, double* x, int
                                     double* bytes_host, int max_kernels, int* count) {
   if (!s || !b || !x || iters <= 0) return GB_BAD_INPUT;
   const size_t bytes = sizeof(double) * s->n;
+  if (precision < 0 || precision > 2) return GB_BAD_INPUT;
   GB_TRY(system_ensure_hist(s, iters + 16));
+  GB_TRY(system_reset_waits(s, precision));
   GB_CUDA_TRY(cudaMemcpyAsync(s->b_int, b, bytes, cudaMemcpyDeviceToDevice, s->s));
   GB_CUDA_TRY(cudaMemcpyAsync(s->v64.x, x, bytes, cudaMemcpyDeviceToDevice, s->s));
   PcgState init;
@@ -204,7 +206,6 @@ extern "C" int gb_profile_iteration(gb_system s, const double* b, double* x, int
   init.hist_len = s->hist_cap;
   init.flag = 1;
   PcgState* st = s->st;
-  if (precision < 0 || precision > 2) return GB_BAD_INPUT;
   if (precision == 0) {
     GB_CUDA_TRY(cudaMemcpyAsync(st, &init, sizeof init, cudaMemcpyHostToDevice, s->s));
     GB_TRY(launch_prologue<double>(s, st, 0, s->b_int));
@@ -244,6 +245,9 @@ extern "C" int gb_profile_iteration(gb_system s, const double* b, double* x, int
     }
   }
   if (rc != GB_OK) return rc;
+  int err = 0;
+  GB_CUDA_TRY(cudaMemcpy(&err, s->err, sizeof(int), cudaMemcpyDeviceToHost));
+  if (err) return err;  // a wait gave up: its kernel's time says nothing
   std::string names;
   const int outk = std::min(nk, max_kernels);
   for (int k = 0; k < outk; ++k) {

@@ -638,6 +638,17 @@ static int read_state(gb_system s, PcgState* dst, const PcgState* src) {
   return GB_OK;
 }
 
+namespace gb {
+int system_reset_waits(gb_system s, int precision) {
+  GB_CUDA_TRY(cudaMemsetAsync(s->err, 0, sizeof(int), s->s));
+  for (TriPlan* p : {precision == 0 ? &s->L : &s->L32, precision == 0 ? &s->U : &s->U32}) {
+    GB_TRY(step_plan_reset(&p->step, s->s));
+    GB_TRY(flow_plan_reset(&p->flow, s->s));
+  }
+  return GB_OK;
+}
+}  // namespace gb
+
 // Core solve on the internal buffers b_int (rhs) and v64.x (x0 -> x).
 static int solve_internal(gb_system s, const gb_pcg_opts* oin, gb_pcg_result* res, double* hist_host,
                           int hist_len) {
@@ -645,11 +656,7 @@ static int solve_internal(gb_system s, const gb_pcg_opts* oin, gb_pcg_result* re
   if (oc.precision < 0) oc.precision = s->auto_precision;  // the autotuner's choice
   const gb_pcg_opts* o = &oc;
   GB_TRY(system_ensure_hist(s, o->maxit));
-  GB_CUDA_TRY(cudaMemsetAsync(s->err, 0, sizeof(int), s->s));
-  for (TriPlan* p : {o->precision == 0 ? &s->L : &s->L32, o->precision == 0 ? &s->U : &s->U32}) {
-    GB_TRY(step_plan_reset(&p->step, s->s));
-    GB_TRY(flow_plan_reset(&p->flow, s->s));
-  }
+  GB_TRY(system_reset_waits(s, o->precision));
   gb_pcg_result r;
   memset(&r, 0, sizeof r);
   PcgState* hs = s->st_host;

@@ -102,5 +102,8 @@ struct gb_system_s {
 
 namespace gb {
 int system_ensure_hist(gb_system sys, int maxit);
+// The error word and what the triangular solves' waits go by, as before any
+// solve: a launch that timed out leaves values behind.
+int system_reset_waits(gb_system sys, int precision);
 void batch_release(gb_batch bt);
 }
