@@ -277,7 +277,8 @@ int gb_debug_flow_plan(int n, const int *ia_host, const int *ja_host, int lower,
  * of one PCG iteration's kernels, averaged over `iters` iterations run
  * eagerly.  names_host receives a ';'-separated list of kernel names,
  * ms_host[i] and bytes_host[i] the average time and algorithmic bytes.
- * GB_TIMEOUT where a wait of one of them gave up. */
+ * A recurrence that runs as one launch is one entry, "team", with its time an
+ * iteration.  GB_TIMEOUT where a wait of one of them gave up. */
 int gb_profile_iteration(gb_system sys, const double *b, double *x, int precision, int iters,
                          char *names_host, int names_len, double *ms_host,
                          double *bytes_host, int max_kernels, int *count);

@@ -598,24 +598,27 @@ static int run_recurrence_split(gb_system s, double tol, int maxit, const double
   return run_loop(s, 2, &launch_body_split, maxit, use_graph);
 }
 
+namespace gb {
+int system_team_loop(gb_system s, int precision) {
+  if (!s->team.on || precision > 1) return GB_NOT_SUPPORTED;
+  const bool jac = s->prec == GB_PREC_LINE_JACOBI;
+  if (precision == 0) {
+    auto& v = s->v64;
+    TeamData<double, double> d{s->ia, s->ja, s->a,    jac ? s->d_r : nullptr, v.x, v.r, jac ? v.w : v.r, v.p0, v.q,
+                               nullptr, s->n, s->st, s->hist, 1, s->err};
+    return team_loop(s->team, d, s->s);
+  }
+  auto& v = s->v32;
+  TeamData<float, float> d{s->ia, s->ja, s->a32,  jac ? s->d_r32 : nullptr, v.x, v.r, jac ? v.w : v.r, v.p0, v.q,
+                           nullptr, s->n, s->st, s->hist, 1, s->err};
+  return team_loop(s->team, d, s->s);
+}
+}  // namespace gb
+
 // Runs (or resumes) the iteration loop until the recurrence's done flag.
 static int run_loop(gb_system s, int idx, BodyFn body_fn, int maxit, int use_graph) {
-  if (s->team.on && idx < 2) {  // one launch, captured or not; the loop where the device refuses it
-    const bool jac = s->prec == GB_PREC_LINE_JACOBI;
-    int rc = GB_OK;
-    if (idx == 0) {
-      auto& v = s->v64;
-      TeamData<double, double> d{s->ia, s->ja, s->a,    jac ? s->d_r : nullptr, v.x, v.r, jac ? v.w : v.r, v.p0, v.q,
-                                 nullptr, s->n, s->st, s->hist, 1, s->err};
-      rc = team_loop(s->team, d, s->s);
-    } else {
-      auto& v = s->v32;
-      TeamData<float, float> d{s->ia, s->ja, s->a32,  jac ? s->d_r32 : nullptr, v.x, v.r, jac ? v.w : v.r, v.p0, v.q,
-                               nullptr, s->n, s->st, s->hist, 1, s->err};
-      rc = team_loop(s->team, d, s->s);
-    }
-    if (rc != GB_NOT_SUPPORTED) return rc;
-  }
+  const int rc = system_team_loop(s, idx);  // one launch, captured or not
+  if (rc != GB_NOT_SUPPORTED) return rc;
   if (use_graph) {
     LoopGraph* lg = nullptr;
     GB_TRY(get_loop_graph(s, idx, body_fn, &lg));

@@ -105,5 +105,8 @@ int system_ensure_hist(gb_system sys, int maxit);
 // The error word and what the triangular solves' waits go by, as before any
 // solve: a launch that timed out leaves values behind.
 int system_reset_waits(gb_system sys, int precision);
+// The recurrence as one launch from the system's state, where it fits the
+// device; GB_NOT_SUPPORTED where it does not or the launch is refused.
+int system_team_loop(gb_system sys, int precision);
 void batch_release(gb_batch bt);
 }

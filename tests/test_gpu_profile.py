@@ -1,4 +1,5 @@
-"""gb_profile_iteration on a system whose solves' waits run out, and after it."""
+"""gb_profile_iteration: what it reports is what solves run, also where the
+recurrence is one launch, and on a system whose waits run out."""
 import numpy as np
 import pytest
 
@@ -37,4 +38,28 @@ def test_waits_that_run_out(precision):
     assert [k["name"] for k in s.profile(b, precision=precision, iters=2)] == names
     again, r = s.solve(b, **kw)
     assert r["status"] == 0 and torch.equal(again, x)
+    s.close()
+
+
+@pytest.mark.parametrize("prec", ["line_jacobi", "none"])
+def test_one_launch_recurrence(prec):
+    """256 x 256 runs whole in one launch: one entry, whose time is that of a
+    solve's iteration (two timings of the same loop, the least of three each,
+    within a quarter; the loop's own kernels took twice as long).  700 x 700
+    does not fit the device and runs them."""
+    A, b = gen.grid2d_unit(256, seed=1001)
+    b = torch.from_numpy(b).cuda()
+    s = gb.System.from_csr(A, prec)
+    for precision in (0, 1):
+        runs = [s.profile(b, precision=precision, iters=500) for _ in range(3)]
+        assert [[k["name"] for k in r] for r in runs] == [["team"]] * 3
+    ms = min(s.profile(b, precision=0, iters=500)[0]["ms"] for _ in range(3))
+    run = min(r["device_ms"] / r["iters"] for _, r in (s.solve(b, tol=0.0, maxit=500) for _ in range(3)))
+    assert 0.75 < ms / run < 1.25
+    x, r = s.solve(b, tol=1e-10, maxit=5000)
+    assert r["status"] == 0 and r["flag"] == 0
+    s.close()
+    A, b = gen.grid2d_unit(700, seed=1001)
+    s = gb.System.from_csr(A, prec)
+    assert [k["name"] for k in s.profile(torch.from_numpy(b).cuda(), iters=4)] == ["spmv_pq", "update"]
     s.close()
