@@ -188,13 +188,13 @@ void free_set(RecordSet* rs) {
 
 }  // namespace
 
-// A record form asked for through its own settings keeps the records.
-static bool record_form_forced() {
-  for (const char* e : {"GBLAP_TRI_FORM", "GBLAP_TRI_SHORT", "GBLAP_TRI_FIXED", "GBLAP_TRI_CLUSTER",
-                        "GBLAP_TRI_FP64_CLUSTER", "GBLAP_TRI_TILE_ROWS", "GBLAP_TRI_TILE_ROWS32",
+// A record form asked for through its own settings keeps the records of the
+// precision that the setting speaks of.
+static bool record_form_forced(int elem) {
+  for (const char* e : {"GBLAP_TRI_FORM", "GBLAP_TRI_SHORT", "GBLAP_TRI_CLUSTER", "GBLAP_TRI_TILE_ROWS",
                         "GBLAP_TRI_BLOCKS_PER_SM", "GBLAP_TRI_LEVEL_RUN", "GBLAP_TRI_PART_DEPS"})
     if (getenv(e)) return true;
-  return false;
+  return elem == 4 ? getenv("GBLAP_TRI_FIXED") || getenv("GBLAP_TRI_TILE_ROWS32") : getenv("GBLAP_TRI_FP64_CLUSTER") != nullptr;
 }
 
 // Global levels (dependency depth) of the rows; returns their number.
@@ -277,7 +277,7 @@ static int form_without_step(const TriDeps& d, int nlev, bool step_fits) {
 // 115, 200k-row kNN 86 / 69 -> 62 / 45, 27-point 64^3 1510 / 1525 -> 490 / 383,
 // a band of 12 on 4000 rows 5148 / 6096 -> 2675 / 2067.
 int tri_step_plan_build(const TriDeps& d, TriPlan* plan, int elem) {
-  if (record_form_forced()) return GB_OK;
+  if (record_form_forced(elem)) return GB_OK;
   std::vector<int> lev;
   const int nlev = row_levels(d, &lev);
   GB_TRY(step_plan_build(d, lev, nlev, elem, flow_estimate(d.n, nlev, elem), &plan->step));
@@ -731,6 +731,8 @@ int tri_solve_plain(const TriPlan* p, const double* x, double* y, int* err, cuda
 
 extern "C" int gb_debug_tri_form(int n, const int* ia_host, const int* ja_host, int lower, int elem_bytes, int* form) {
   if (n <= 0 || !ia_host || !ja_host || !form || (elem_bytes != 4 && elem_bytes != 8)) return GB_BAD_INPUT;
+  *form = gb::kFormRecords;
+  if (gb::record_form_forced(elem_bytes)) return GB_OK;
   const gb::TriDeps d = gb::deps_of_part(n, ia_host, ja_host, lower != 0);
   std::vector<int> lev;
   const int nlev = gb::row_levels(d, &lev);

@@ -107,6 +107,18 @@ def test_form(name):
     assert forms(make()) == want
 
 
+@pytest.mark.parametrize("name,want", [
+    ("GBLAP_TRI_FORM", (RECORDS,) * 4),
+    ("GBLAP_TRI_TILE_ROWS", (RECORDS,) * 4),  # the FP32 tile follows it
+    ("GBLAP_TRI_TILE_ROWS32", (STEP, STEP, RECORDS, RECORDS)),
+    ("GBLAP_TRI_FIXED", (STEP, STEP, RECORDS, RECORDS)),
+    ("GBLAP_TRI_FP64_CLUSTER", (RECORDS, RECORDS, STEP, STEP)),
+])
+def test_a_setting_keeps_the_records_it_speaks_of(name, want, monkeypatch):
+    monkeypatch.setenv(name, "1024")
+    assert forms(box(20, 20, 20)) == want
+
+
 def test_bad_input():
     A = path(4)
     f = np.zeros(1, np.int32)
