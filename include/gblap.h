@@ -249,6 +249,12 @@ int gb_debug_set_spin_budget(gb_system sys, unsigned long long ns);
  * the solve runs the captured loop instead. */
 int gb_debug_set_team_smem(gb_system sys, gb_batch batch, int bytes);
 
+/* Test hooks: a block of those launches that leaves at once, without a word to
+ * its team (-1: none), so that the team's waits run out and the solve ends with
+ * GB_TIMEOUT; and gb_debug_set_spin_budget for a batch. */
+int gb_debug_set_team_silent(gb_system sys, gb_batch batch, int block);
+int gb_debug_set_batch_spin_budget(gb_batch batch, unsigned long long ns);
+
 /* Test hook (host only): the lock-step solve plan of the strict lower / upper
  * part of a full CSR pattern, for values of elem_bytes (4 or 8).  tile_rows 0:
  * the planner's choice.  info: {tiles, rows of a tile, solver warps, staged

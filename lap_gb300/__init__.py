@@ -109,6 +109,8 @@ def _proto(L: C.CDLL) -> None:
         "gb_pcg_autotune_precision": (i, [vp, vp, vp, C.POINTER(i), vp]),
         "gb_debug_set_spin_budget": (i, [vp, C.c_ulonglong]),
         "gb_debug_set_team_smem": (i, [vp, vp, i]),
+        "gb_debug_set_team_silent": (i, [vp, vp, i]),
+        "gb_debug_set_batch_spin_budget": (i, [vp, C.c_ulonglong]),
         "gb_debug_step_plan": (i, [i, vp, vp, i, i, i, vp, vp, vp, vp, vp, vp, vp]),
         "gb_debug_tri_form": (i, [i, vp, vp, i, i, vp]),
         "gb_debug_flow_plan": (i, [i, vp, vp, i, vp, vp, vp, vp, vp, vp]),

@@ -1077,7 +1077,7 @@ int batch_buffers(gb_batch bt) {
   for (double** v : {&bt->b, &bt->x, &bt->r, &bt->w, &bt->p, &bt->q}) GB_TRY(balloc(bt, v, N));
   if (bt->inter) GB_TRY(balloc(bt, &bt->w32, N));
   if (bt->inter) GB_TRY(balloc(bt, &bt->rep, bt->count));
-  GB_TRY(balloc(bt, &bt->st, bt->count));
+  GB_TRY(balloc(bt, &bt->st, bt->count + 1));
   GB_TRY(balloc(bt, &bt->so, bt->count));
   GB_CUDA_TRY(cudaMallocHost(&bt->st_h, sizeof(PcgState) * 2 * bt->count));
   GB_TRY(batch_parts(bt));
@@ -1411,6 +1411,17 @@ extern "C" int gb_batch_create(int count, const long long* row_off_host, const l
 extern "C" int gb_debug_set_team_smem(gb_system sys, gb_batch bt, int bytes) {
   if ((!sys && !bt) || bytes < 0 || (size_t)bytes > kTeamMaxSmem) return GB_BAD_INPUT;
   (sys ? sys->team : bt->team).debug_smem = (size_t)bytes;
+  return GB_OK;
+}
+
+extern "C" int gb_debug_set_team_silent(gb_system sys, gb_batch bt, int block) {
+  if (!sys && !bt) return GB_BAD_INPUT;
+  return sys ? team_debug_silent(&sys->team, block, sys->st) : team_debug_silent(&bt->team, block, bt->st);
+}
+
+extern "C" int gb_debug_set_batch_spin_budget(gb_batch bt, unsigned long long ns) {
+  if (!bt || !bt->err) return GB_BAD_INPUT;
+  GB_CUDA_TRY(cudaMemcpy(bt->err + 2, &ns, sizeof ns, cudaMemcpyHostToDevice));
   return GB_OK;
 }
 

@@ -417,12 +417,14 @@ int team_plan_build(int count, const std::vector<int>& row_off, const int* ia, T
   }
   p->rows = rows;
   p->ctas = (int)c;
+  p->systems = count;
   p->smem = (size_t)p->max_nnz * (sizeof(double) + sizeof(int));
   if (p->smem > kTeamMaxSmem || resident(rows, p->smem) < p->ctas) {
     p->smem = 0;
     if (resident(rows, 0) < p->ctas) return GB_OK;
   }
   GB_TRY(to_device(&p->cta_sys, cta_sys));
+  cta0.push_back(cta0.back());
   GB_TRY(to_device(&p->cta0, cta0));
   GB_TRY(to_device(&p->mail0, mail0));
   GB_CUDA_TRY(cudaMalloc(&p->mail, sizeof(double) * p->mail_len));
@@ -434,6 +436,20 @@ void team_plan_free(TeamPlan* p) {
   for (void* q : {(void*)p->cta_sys, (void*)p->cta0, (void*)p->mail, (void*)p->mail0})
     if (q) cudaFree(q);
   *p = TeamPlan();
+}
+
+int team_debug_silent(TeamPlan* p, int block, PcgState* states) {
+  if (!p->on || block >= p->ctas) return GB_BAD_INPUT;
+  if (p->debug_block >= 0)
+    GB_CUDA_TRY(cudaMemcpy(p->cta_sys + p->debug_block, &p->debug_sys, sizeof(int), cudaMemcpyHostToDevice));
+  p->debug_block = -1;
+  if (block < 0) return GB_OK;
+  const int one = 1;
+  GB_CUDA_TRY(cudaMemcpy(&states[p->systems].done, &one, sizeof(int), cudaMemcpyHostToDevice));
+  GB_CUDA_TRY(cudaMemcpy(&p->debug_sys, p->cta_sys + block, sizeof(int), cudaMemcpyDeviceToHost));
+  GB_CUDA_TRY(cudaMemcpy(p->cta_sys + block, &p->systems, sizeof(int), cudaMemcpyHostToDevice));
+  p->debug_block = block;
+  return GB_OK;
 }
 
 template <typename T, typename TA>

@@ -18,7 +18,9 @@ struct TeamPlan {
   size_t smem = 0;          // bytes of matrix entries kept in shared memory (0: none)
   int max_nnz = 0;          // most entries of a block
   size_t debug_smem = 0;    // test hook: bytes to ask for at least, past what the device gives every block
-  int *cta_sys = nullptr, *cta0 = nullptr;  // device [ctas], [systems + 1]
+  int systems = 0;
+  int *cta_sys = nullptr, *cta0 = nullptr;  // device [ctas], [systems + 2] (the last twice)
+  int debug_block = -1, debug_sys = 0;      // test hook: a block that leaves at once, and its system
   double *mail = nullptr;        // device: per system [blocks][4][blocks][2]
   long long *mail0 = nullptr;    // device [systems]
   long long mail_len = 0;
@@ -33,6 +35,9 @@ constexpr int kTeamMaxRow = 64;  // entries of a row (a thread sums its rows alo
 // at once and no row is too long.
 int team_plan_build(int count, const std::vector<int>& row_off, const int* ia, TeamPlan* plan);
 void team_plan_free(TeamPlan* plan);
+// Test hook: block `block` (-1: none) belongs to a system past the last whose
+// state, states[systems], is done, and leaves at once without a word to its team.
+int team_debug_silent(TeamPlan* plan, int block, PcgState* states);
 
 // Vectors and matrix of the systems, concatenated; columns local to the
 // system.  d_r null: no preconditioner (w is r).
@@ -44,7 +49,7 @@ struct TeamData {
   T *x, *r, *w, *p, *q;
   const int* row_off;  // null: one system from row 0
   int n;               // rows in all
-  PcgState* st;        // [systems]
+  PcgState* st;        // [systems], and one more for the test hook
   double* hist;        // one system: residual history (st->hist_len entries), or null
   int roll_done;       // rho rolls in the last iteration too (the single-system recurrence's convention)
   int* err;
