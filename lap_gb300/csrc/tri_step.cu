@@ -105,6 +105,11 @@ double step_cycles(int elem, int width) {
 constexpr double kHopCycles = 250.0;      // more for a step whose inputs come from the previous tile
 constexpr double kCrossCycles = 2000.0;   // and from another cluster, through L2
 constexpr int kResidentTiles = 140;       // about what clusters of 8 to 16 place on 152 SMs
+// Seconds a resident tile may wait for the one before it, by the estimate: a
+// wait ends at one second (kSpinBudgetNs).  A path of 9M rows, FP64, in the
+// tallest tiles there are is 146 of 61,697 steps, all running, and the last
+// would wait 1.1 s.
+constexpr double kStepMaxWait = 0.4;
 
 // Tiles of a cluster, as far as can be said before the device is asked.
 int cluster_guess(int ntiles) { return ntiles <= 16 ? ntiles : ntiles <= 112 ? 16 : 10; }
@@ -172,7 +177,8 @@ std::vector<int> step_heights(const TriDeps& d, const std::vector<int>& lev, int
     // clusters that are not resident start when an earlier one has ended
     // (1000 x 700 FP32: 175 tiles 328 us, 88 tiles 189 us)
     cost *= (nt + kResidentTiles - 1) / kResidentTiles;
-    cands.push_back({rows, cost});
+    const double chain = std::min<double>(nlev, (double)std::min(nt, kResidentTiles) * span);
+    if (chain * step_cycles(elem, std::min(width, 32 * kStepMaxWarps)) < kStepMaxWait * 2e9) cands.push_back({rows, cost});
     if (whole) break;
   }
   std::stable_sort(cands.begin(), cands.end(), [](const Cand& a, const Cand& b) { return a.cost < b.cost; });
