@@ -262,7 +262,8 @@ int gb_debug_set_batch_spin_budget(gb_batch batch, unsigned long long ns);
  * natural order, chunks}.
  * The arrays (NULL: sizes only): tiles [8 per tile] {row0, rows, page0, pages,
  * step0, steps, exports, first chunk}, ends [steps], meta [pages * 128 * 4], src
- * [pages * 128 * 4], needs [pages], thr [chunks].  GB_NOT_SUPPORTED where the factor keeps its records. */
+ * [pages * 128 * 4], needs [pages], thr [chunks].  GB_NOT_SUPPORTED where the factor
+ * leaves no room for it; whether it is also run gb_debug_tri_form says. */
 int gb_debug_step_plan(int n, const int *ia_host, const int *ja_host, int lower, int elem_bytes, int tile_rows,
                        int *info, int *tiles, unsigned short *ends, unsigned *meta, int *src,
                        unsigned short *needs, unsigned short *thr);

@@ -118,8 +118,8 @@ struct EpAxpby {
 
 // y = alpha A x + beta y in the reference's order and rounding.  FP64 is bound
 // by its pipe: a multiply and an add per entry (two multiplies unless UNIT) at
-// 64 cycles a warp are 47 us on 128^3, the bytes 32 us.  Measured with the
-// call's launch and synchronisation (~10 us), 128^3: 119.5 -> 84.9 us at
+// 64 cycles a warp are 47 us on 128^3, the bytes 32 us.  Measured through
+// gb_spmv, whose launch and synchronisation are 12 us, 128^3: 119.5 -> 84.4 us at
 // alpha = 1 (one multiply less, rows read per lane instead of staged, no
 // comparison of beta, the next bundle's head in flight, four blocks an SM:
 // five 86.8, six 90.9), 114 us otherwise.

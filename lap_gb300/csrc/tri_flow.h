@@ -1,5 +1,5 @@
-// tri_flow.h -- plan of the triangular solves of every factor that the
-// lock-step form does not take (tri_flow.cuh has the kernel and its reasons).
+// tri_flow.h -- plan of the value-polling triangular solves (tri_flow.cuh has
+// the kernel and its reasons, tri_plan.cu which factors take them).
 #pragma once
 
 #include <vector>
