@@ -44,7 +44,9 @@ struct SpmvPlan {
   int n = 0, nnz = 0;
   int nbundles = 0;
   int *bundles = nullptr;   // device [nbundles+1]
-  int longest = 0;          // entries of the longest row
+  // whether the kernels that sum long rows by the whole warp gain, FP64 / FP32
+  // products (spmv_bundle.cuh)
+  bool long64 = false, long32 = false;
   int rows_per_bundle = kBundleRows;
 };
 

@@ -83,7 +83,33 @@ int spmv_plan_build(int n, int nnz, const int* ia, SpmvPlan* plan, int rpb) {
   plan->n = n;
   plan->nnz = nnz;
   plan->nbundles = (int)b.size() - 1;
-  plan->longest = longest;
+  // FP64 products gain wherever a row is long or lose nothing.  FP32 ones lose
+  // 3 to 10% to the kernel's fewer resident blocks where nothing is summed so
+  // (rows of 33, 61, 101: 25.3 -> 26.5, 44 -> 46, 81 -> 91 us), so they take it
+  // where a row is too long to stage, a fifth of the summing goes away or the
+  // slowest bundle halves (125 entries a row 37 -> 30 us, 201 68 -> 35, one row
+  // of 400 in 100^3 30 -> 24).
+  plan->long64 = longest > kSpmvSerial;
+  plan->long32 = longest > cap;
+  if (plan->long64 && !plan->long32) {
+    long long serial = 0, best = 0;
+    int slowest = 0, slowest_best = 0;
+    for (size_t i = 0; i + 1 < b.size(); ++i) {
+      int most = 0, rest = 0, rows = 0;
+      for (int j = b[i]; j < b[i + 1]; ++j) {
+        const int len = ia[j + 1] - ia[j];
+        most = std::max(most, len);
+        if (len > kSpmvSerial) ++rows;
+        else rest = std::max(rest, len);
+      }
+      const int by_warp = rows * (int)kSpmvRowCost<float>, cost = rows && by_warp <= most ? by_warp + rest : most;
+      serial += most;
+      best += cost;
+      slowest = std::max(slowest, most);
+      slowest_best = std::max(slowest_best, cost);
+    }
+    plan->long32 = 5 * best < 4 * serial || 2 * slowest_best < slowest;
+  }
   plan->rows_per_bundle = rpb;
   // every bundle 32 consecutive rows (a stencil): the kernels' plan-free
   // layout computes the same bundles, one dependent load fewer per bundle.

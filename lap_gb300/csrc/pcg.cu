@@ -130,8 +130,7 @@ __global__ void __launch_bounds__(kThreads)
 // Five resident blocks per SM, as spmv_pq_split_kernel: the FP64 form then
 // holds 48 registers with a 72-byte spill instead of 64 (128^3: 69.0 ->
 // 62.4 us); the FP32 form needs 48 either way.
-// LONG, for a matrix with a row of more than kSpmvSerial entries, needs more
-// registers and runs four.
+// LONG (SpmvPlan::long64, long32) needs more registers and runs four.
 template <typename T, int WK, bool LONG>
 __global__ void __launch_bounds__(kThreads, LONG ? 4 : 5)
     spmv_pq_kernel(int n, int nb, const int* __restrict__ bundles, const int* __restrict__ ia,
@@ -821,7 +820,7 @@ int launch_body_split(gb_system sys, PcgState* st, cudaGraphConditionalHandle co
   auto& v = sys->v64;
   const int nb = sys->plan.nbundles;
   const float* w = sys->prec == GB_PREC_ICHOL ? sys->v32.s : sys->v32.w;
-  const bool rows_long = sys->plan.longest > kSpmvSerial;
+  const bool rows_long = sys->plan.long32;
   auto pq = rows_long ? spmv_pq_split_kernel<true> : spmv_pq_split_kernel<false>;
   pq<<<rows_long ? std::min(grid_split(nb), wave_grid(pq, kThreads, ceil_div(nb, kThreads / 32))) : grid_split(nb), kThreads, 0, sys->s>>>(
       sys->n, nb, sys->plan.bundles, sys->ia, sys->ja, sys->a32, w, v.p0, v.q,
@@ -870,7 +869,7 @@ int launch_body(gb_system sys, PcgState* st, cudaGraphConditionalHandle cond, in
   const T* a = mat_vals<T>(sys);
   const T* dr = dr_vals<T>(sys);
   const T* wbuf = w_buffer<T>(sys);
-  const bool rows_long = sys->plan.longest > kSpmvSerial;
+  const bool rows_long = sizeof(T) == 8 ? sys->plan.long64 : sys->plan.long32;
 #define GB_PQ(WKV)                                                                             \
   do {                                                                                         \
     auto pq = rows_long ? spmv_pq_kernel<T, WKV, true> : spmv_pq_kernel<T, WKV, false>;        \

@@ -51,14 +51,21 @@ __device__ __forceinline__ void ep_prefetch(EP&, int, long) {}
 // Values of a row held in registers from the start of its bundle (FMA
 // form): a stencil row's whole dependency list is in flight at once.
 constexpr int kSpmvHeld = 8;
-// LONG (FMA form), for matrices with rows of more than kSpmvSerial entries:
-// entries a lane sums by itself at most, and gathers of a lane in flight in a
-// row too long to stage.  131k-row Chung-Lu (a row of 11k entries), one
+// LONG (FMA form), for matrices with rows of more than kSpmvSerial entries: the
+// whole warp sums such a row, and keeps kSpmvBatch gathers of a lane in flight
+// in a row too long to stage.  131k-row Chung-Lu (a row of 11k entries), one
 // spmv_pq: 118 -> 67 us in FP64, 59 -> 34 us in split precision; 3k rows 40 ->
 // 21 us.  Bound by the longest row's chain of gathers.  A kernel of its own:
 // in the others its registers would spill (FP64 spmv_pq 72 -> 260 bytes).
+// A row summed so costs the warp about as much as kSpmvRowCost entries summed
+// by a lane, which the lanes' other rows share: a bundle's long rows are summed
+// so where that is less than its longest.  (Every row of 33: 50 us serial, 183
+// by the warp, 48 so; of 101: 272 -> 211; of 401: 466 -> 49; kNN rows of up to
+// 50: 71, 153, 64; FP64.)  SpmvPlan::long32 says where it gains in FP32.
 constexpr int kSpmvSerial = 32;
 constexpr int kSpmvBatch = 8;
+template <typename T>
+constexpr unsigned kSpmvRowCost = sizeof(T) == 8 ? 12u : 24u;
 // 1: bundles whose rows all have at most kSpmvHeld entries take the
 // per-lane form (no staging).
 #ifndef GB_SPMV_SHORT_ROWS
@@ -236,6 +243,8 @@ __device__ __forceinline__ void spmv_bundle_h(const BundleHead& h, const int* __
   bool mine = own;
   if constexpr (LONG) {
     unsigned lng = __ballot_sync(0xffffffffu, own && re - rs > kSpmvSerial);
+    if (lng != 0u && __popc(lng) * kSpmvRowCost<T> >
+                         __reduce_max_sync(0xffffffffu, own ? (unsigned)(re - rs) : 0u)) lng = 0u;
     if (lng & (1u << lane)) mine = false;
     while (lng) {
       const int src = __ffs(lng) - 1;
