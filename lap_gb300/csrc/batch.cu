@@ -1185,7 +1185,7 @@ int batch_loop(gb_batch bt, int split, int maxit, int use_graph) {
                                bt->row_off, bt->N, bt->st, nullptr, 0, bt->err};
     TeamData<double, float> f{d.ia, d.ja, bt->a32, d.d_r, d.x, d.r, d.w, d.p, d.q, d.row_off, d.n, d.st, nullptr, 0, d.err};
     const int rc = split ? team_loop(bt->team, f, bt->s) : team_loop(bt->team, d, bt->s);
-    if (rc != GB_NOT_SUPPORTED) return rc;  // the loop where the device refuses the launch
+    if (rc != GB_NOT_SUPPORTED) return rc;  // the loop where that is faster or the launch refused
   }
   GB_CUDA_TRY(cudaMemsetAsync(bt->tk, 0, sizeof(unsigned) * 4, bt->s));
   GB_CUDA_TRY(cudaMemsetAsync(bt->nactive, 0, sizeof(int) * 4, bt->s));
@@ -1626,7 +1626,7 @@ extern "C" int gb_batch_autotune(gb_batch bt, const double* b, int iters, int* r
   if (iters <= 0) iters = 16;
   int maxrow = 0;
   for (int i = 0; i < bt->N; ++i) maxrow = std::max(maxrow, bt->h_ia[i + 1] - bt->h_ia[i]);
-  const BatchClass key{bt->count, bt->N, bt->h_ia[bt->N], maxrow, bt->team.on};
+  const BatchClass key{bt->count, bt->N, bt->h_ia[bt->N], maxrow, team_runs<double, double>(bt->team, true)};
   std::pair<int, int> best{kBundleRows, kChunkRows};
   double t_def = 0.0, t_best = 0.0;
   bool cached = false;
@@ -1645,7 +1645,7 @@ extern "C" int gb_batch_autotune(gb_batch bt, const double* b, int iters, int* r
     t_best = 1e300;
     for (int rpb : {kBundleRows, 16, 8}) {
       for (int cr : {kChunkRows, 1024, 4096}) {
-        if (bt->team.on && (rpb != kBundleRows || cr != kChunkRows)) continue;
+        if (key.team && (rpb != kBundleRows || cr != kChunkRows)) continue;
         double ms = 0.0;
         rc = batch_replan(bt, rpb, cr);
         if (rc == GB_OK) rc = batch_time(bt, b, x, iters, &ms);

@@ -600,7 +600,7 @@ static int run_recurrence_split(gb_system s, double tol, int maxit, const double
 
 namespace gb {
 int system_team_loop(gb_system s, int precision) {
-  if (!s->team.on || precision > 1) return GB_NOT_SUPPORTED;
+  if (precision > 1) return GB_NOT_SUPPORTED;
   const bool jac = s->prec == GB_PREC_LINE_JACOBI;
   if (precision == 0) {
     auto& v = s->v64;

@@ -418,6 +418,7 @@ int team_plan_build(int count, const std::vector<int>& row_off, const int* ia, T
   p->rows = rows;
   p->ctas = (int)c;
   p->systems = count;
+  p->nnz = (long long)ia[n] - ia[0];
   p->smem = (size_t)p->max_nnz * (sizeof(double) + sizeof(int));
   if (p->smem > kTeamMaxSmem || resident(rows, p->smem) < p->ctas) {
     p->smem = 0;
@@ -454,6 +455,7 @@ int team_debug_silent(TeamPlan* p, int block, PcgState* states) {
 
 template <typename T, typename TA>
 int team_loop(const TeamPlan& p, const TeamData<T, TA>& d, cudaStream_t s) {
+  if (!team_runs<T, TA>(p, d.hist == nullptr)) return GB_NOT_SUPPORTED;
   GB_TRY(fill_sentinel_dev((int)p.mail_len, p.mail, s));
   TeamArgs<T, TA> A;
   A.d = d;

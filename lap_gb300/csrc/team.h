@@ -17,6 +17,7 @@ struct TeamPlan {
   int ctas = 0, rows = 0;   // blocks; rows of a thread (1 to 4)
   size_t smem = 0;          // bytes of matrix entries kept in shared memory (0: none)
   int max_nnz = 0;          // most entries of a block
+  long long nnz = 0;        // entries in all
   size_t debug_smem = 0;    // test hook: bytes to ask for at least, past what the device gives every block
   int systems = 0;
   int *cta_sys = nullptr, *cta0 = nullptr;  // device [ctas], [systems + 2] (the last twice)
@@ -55,11 +56,25 @@ struct TeamData {
   int* err;
 };
 
+// Whether the one launch is the faster way: past these entries the loops' kernels,
+// which stage rows by whole lines, win over threads that read their own rows.
+// An iteration, loop -> one launch, us.  FP64, one system: 27-point 70^3 (9.0M
+// entries) 88 -> 82, 74^3 (10.6M) 94 -> 106, a band of 25 on 400k rows (10.0M)
+// 89 -> 97; a batch's loop has four launches: 109 -> 97, a band of 33 there
+// (13.2M) 139 -> 140, split 117 -> 132, and 10.0M 95 -> 85.  FP32: a band of 25 on
+// 200k rows (5.0M) 43 -> 37, random 12 on 400k (5.2M) 60 -> 60, a band of 33
+// (6.6M) 47 -> 53.
+template <typename T, typename TA>
+bool team_runs(const TeamPlan& plan, bool batch) {
+  const long long most = sizeof(T) == 4 ? 5000000 : sizeof(TA) == 4 ? 10000000 : batch ? 12000000 : 9000000;
+  return plan.on && plan.nnz <= most;
+}
+
 // Runs every system's recurrence from its state until it is done (or its
 // state says it is), as the loops of update / spmv_pq kernels do.
-// GB_NOT_SUPPORTED, with nothing of the state touched, where the device refuses
-// the launch (fewer SMs for this context than when the plan was made): the
-// caller then runs the loop.
+// GB_NOT_SUPPORTED, with nothing of the state touched, where it is not the
+// faster way or the device refuses the launch (fewer SMs for this context than
+// when the plan was made): the caller then runs the loop.
 template <typename T, typename TA>
 int team_loop(const TeamPlan& plan, const TeamData<T, TA>& d, cudaStream_t s);
 
