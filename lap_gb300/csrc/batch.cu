@@ -123,12 +123,21 @@ __device__ __forceinline__ void for_bundles(const BatchArgs& B, F&& body) {
 // [i0, i1), by the whole block; valid in thread 0.  A thread's loads go out
 // eight at a time: one after another they were most of the reduction (80^3,
 // 32 right-hand sides, 6,080 partials each: alpha 20 -> 9, check 23 ->
-// 14 us).
+// 14 us).  Where a thread has no more than two, the guards of the eight cost
+// more than they save (two right-hand sides of 20^3, an iteration: 24.5 us so,
+// 26.0 eight at a time); the sums are the same.
 template <int NV>
 __device__ __forceinline__ void block_segment_sum(const double* part, int stride, int i0, int i1,
                                                   double (&v)[NV], double* sm) {
 #pragma unroll
   for (int k = 0; k < NV; ++k) v[k] = 0.0;
+  if (i1 - i0 <= 2 * (int)blockDim.x) {
+    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x)
+#pragma unroll
+      for (int k = 0; k < NV; ++k) v[k] += part[(size_t)stride * i + k];
+    block_sum<NV>(v, sm);
+    return;
+  }
   constexpr int U = 8;
   for (int i = i0 + threadIdx.x; i < i1; i += U * blockDim.x) {
     double t[U][NV];
