@@ -62,11 +62,11 @@ struct TeamData {
 // entries) 88 -> 82, 74^3 (10.6M) 94 -> 106, a band of 25 on 400k rows (10.0M)
 // 89 -> 97; a batch's loop has four launches: 109 -> 97, a band of 33 there
 // (13.2M) 139 -> 140, split 117 -> 132, and 10.0M 95 -> 85.  FP32: a band of 25 on
-// 200k rows (5.0M) 43 -> 37, random 12 on 400k (5.2M) 60 -> 60, a band of 33
-// (6.6M) 47 -> 53.
+// 200k rows (5.0M) 43 -> 37, random 12 on 400k (5.2M) 60 -> 60, 27-point 60^3
+// (5.6M) 46 -> 42, a band of 33 (6.6M) 47 -> 53.
 template <typename T, typename TA>
 bool team_runs(const TeamPlan& plan, bool batch) {
-  const long long most = sizeof(T) == 4 ? 5000000 : sizeof(TA) == 4 ? 10000000 : batch ? 12000000 : 9000000;
+  const long long most = sizeof(T) == 4 ? 5800000 : sizeof(TA) == 4 ? 10000000 : batch ? 12000000 : 9000000;
   return plan.on && plan.nnz <= most;
 }
 
