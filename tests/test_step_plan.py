@@ -156,17 +156,3 @@ def test_factors_that_keep_their_records():
     far = gen.laplacian_from_edges(200000, np.arange(100000), np.arange(100000, 200000), np.ones(100000), shift=1.0)
     assert plan(far, True, 4) == 8  # the previous tile's exports would not fit beside it
     assert plan(gen.knn_graph(300, rng=rng), True, 4) == 8  # rows of more than four dependencies
-
-
-@pytest.mark.parametrize("elem,step_ns", [(8, 125), (4, 68)])  # as measured on a path of 100,000
-def test_no_tile_waits_a_second(elem, step_ns):
-    """The tiles that run at once wait for one another: their steps together,
-    on a chain as long as they are, take less than half of the second after
-    which a wait gives up."""
-    for n in (3_000_000, 9_000_000):
-        ia = np.clip(3 * np.arange(n + 1) - 1, 0, 3 * n - 2).astype(np.int32)
-        cols = np.arange(n)[:, None] + np.array([-1, 0, 1])
-        ja = cols[(cols >= 0) & (cols < n)].astype(np.int32)
-        info = np.zeros(12, np.int32)
-        assert gb.lib().gb_debug_step_plan(n, ia.ctypes.data, ja.ctypes.data, 1, elem, 0, info.ctypes.data, *[None] * 6) == 0
-        assert min(int(info[0]), 152) * int(info[6]) * step_ns < 0.5e9
